@@ -40,14 +40,31 @@
 //   warps 0-15 epilogue: warp w reads TMEM lanes 32 (w & 3) .. + 31 (its rows
 //             in each row tile) and 16 of a slab's 64 columns (column group
 //             w >> 2); four epilogue warps per SM sub-partition hide the
-//             TMEM-load and shuffle latencies.  Per pair, row sums and column
-//             sums are combined over the warps in shared memory in a fixed
-//             order and stored;
+//             reduce-scatter latencies.  TMEM loads run one row tile ahead of the
+//             exponentials, across slabs and pairs.  Per pair, row sums and
+//             column sums are combined over the warps in shared memory (two
+//             copies, one barrier per pair) in a fixed order and stored;
 //   warp 16   copies: the row block's operands when the row block changes,
 //             the column block's operands per pair (two stages);
 //   warp 17   MMA (lane 0): per TMEM unit (UT row tiles of one slab), 6 MMAs
 //             per row tile into one of 8 / UT buffers, committed to that
 //             buffer's "full" barrier.
+// What bounds it: the MUFU ex2 rate, 16 per clock and SM, is 1.08 ms of the
+// n = 100,000 product (5.03e9 evaluated entries).  An issue-level copy of the
+// epilogue loop (TMEM load, ex2, two packed FMAs per entry pair, reduce-scatter)
+// runs 37 cycles per four entries of a thread against 32 at the MUFU rate; the
+// rest is barriers and hand-offs.  576 threads cap the registers at 96, so the
+// loop is written to stay inside them: x of the next pair goes through shared
+// memory by cp.async instead of registers, the walk is 32-bit, x of the rows is
+// stored as pairs {x, x} (no register copies for the packed FMAs), a buffer is
+// released by one arrival per warp, and no branch surrounds the TMEM loads after
+// an abort.  With the spills and the exposed loads gone the n = 100,000 product
+// takes 1.55 ms instead of 1.91 ms (n = 50,000: 0.41 instead of 0.50; whole calls
+// with packing and finish), the same bits.  Measured and not kept: warp-level MMAs
+// (mma.sync m16n8k16) with the logits in registers and no hand-offs, 1.60 ms -- an
+// MMA holds back the FMAs of its sub-partition, 41 cycles per four entries at best;
+// helper warps or a deferred combine instead of the per-pair barrier, 1.68 and
+// 1.75 ms (registers again); setmaxnreg for the epilogue (the other roles spill).
 // Every wait is bounded; a timeout sets a shared abort flag that every role
 // checks; the CTA then drains its copies and MMAs and frees TMEM.  The
 // epilogue warps keep walking their pairs after an abort (without waits or
@@ -104,10 +121,13 @@ struct K1tCfg {
                        kBarDrain = kBarAccEmpty + kBufs, kNumBars = kBarDrain + 1;
   static constexpr uint32_t kOffA = 0;                        // row operands (hi | lo)
   static constexpr uint32_t kOffB = kOffA + kHalf;            // 2 stages of column operands
+  // per-pair sums: two copies where they fit (one barrier per pair then)
+  static constexpr int kSets = FMT == kK1tTf32 ? 1 : 2;
   static constexpr uint32_t kOffXb = kOffB + 2 * kHalf;       // 2 x 512 floats: x of the column block
-  static constexpr uint32_t kOffRow = kOffXb + 2 * kTB * 4;   // 4 x 512 doubles: row sums per column group
-  static constexpr uint32_t kOffCol = kOffRow + kTNcg * kTB * 8;  // 4 x 512 floats: column sums per row quadrant
-  static constexpr uint32_t kOffBar = kOffCol + 4 * kTB * 4;  // barriers, TMEM slot, abort flag
+  static constexpr uint32_t kOffXa = kOffXb + 2 * kTB * 4;    // 2 x 512 pairs {x, x} of the row block
+  static constexpr uint32_t kOffRow = kOffXa + 2 * kTB * 8;   // sets x 4 x 512 floats: row sums per column group
+  static constexpr uint32_t kOffCol = kOffRow + kSets * kTNcg * kTB * 4;  // sets x 4 x 512: column sums per row quadrant
+  static constexpr uint32_t kOffBar = kOffCol + kSets * 4 * kTB * 4;  // barriers, TMEM slot, abort flag
   static constexpr uint32_t kSmemBytes = kOffBar + kNumBars * 8 + 16 + 1024;  // + alignment slack
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
   static_assert(kSmemBytes > kTmemExclusiveSmem, "one TMEM-owning CTA per SM");
@@ -255,29 +275,30 @@ __global__ void k1t_pack_kernel(const float* __restrict__ packed32, int DP, int6
 }
 
 // A CTA's walk over its pairs (single instance or the running instances of
-// a batch).  `slot` is the pair's index in the partial arrays.
+// a batch).  `slot` is the pair's index in the partial arrays.  32-bit fields:
+// 2^31 pairs would take 13 TB of partial sums (the launchers check).
 struct PairWalk {
-  int64_t p, p_end;
+  int p, p_end;
   int j;
-  int64_t a, b;
-  int64_t nb, npts, seg, pstart, pend, gp0;
+  int a, b;
+  int nb, npts, seg, pstart, pend, gp0;
 
   template <bool BATCHED>
   __device__ __forceinline__ void load_inst(const SymPlan& sp, const BatchMap& bm, int64_t n) {
     if (BATCHED) {
       const SlotInfo& si = bm.slots[bm.act_inst[j]];
-      nb = si.nblk;
-      npts = si.npts;
-      seg = si.seg;
-      pstart = bm.act_ps[j];
-      pend = bm.act_ps[j + 1];
-      gp0 = si.pair_start;
+      nb = (int)si.nblk;
+      npts = (int)si.npts;
+      seg = (int)si.seg;
+      pstart = (int)bm.act_ps[j];
+      pend = (int)bm.act_ps[j + 1];
+      gp0 = (int)si.pair_start;
     } else {
-      nb = sp.nb;
-      npts = n;
+      nb = (int)sp.nb;
+      npts = (int)n;
       seg = 0;
       pstart = 0;
-      pend = sp.npairs;
+      pend = (int)sp.npairs;
       gp0 = 0;
     }
   }
@@ -291,31 +312,38 @@ struct PairWalk {
         load_inst<BATCHED>(sp, bm, n);
       }
     }
-    sym_pair_coords(p - pstart, nb, &a, &b);
+    int64_t aa, bb;
+    sym_pair_coords(p - pstart, nb, &aa, &bb);
+    a = (int)aa;
+    b = (int)bb;
     return true;
   }
   template <bool BATCHED>
   __device__ __forceinline__ bool next(const SymPlan& sp, const BatchMap& bm, int64_t n) {
     ++p;
     if (p >= p_end) return false;
-    if (p < pend) {
-      if (++b >= nb) {
-        ++a;
-        b = a;
-      }
+    if (p >= pend) {  // the next running instance starts at its first pair
+      do {
+        ++j;
+        load_inst<BATCHED>(sp, bm, n);
+      } while (p >= pend);
+      a = b = 0;
       return true;
     }
-    return settle<BATCHED>(sp, bm, n);
+    if (++b >= nb) {
+      ++a;
+      b = a;
+    }
+    return true;
   }
-  __device__ __forceinline__ int64_t slot() const { return gp0 + p - pstart; }
+  __device__ __forceinline__ int64_t slot() const { return gp0 + (p - pstart); }
   // global image blocks of the pair's row and column blocks
-  __device__ __forceinline__ int64_t row_block() const { return seg / kTB + a; }
-  __device__ __forceinline__ int64_t col_block() const { return seg / kTB + b; }
+  __device__ __forceinline__ int row_block() const { return seg / kTB + a; }
+  __device__ __forceinline__ int col_block() const { return seg / kTB + b; }
   // column slabs holding points
   __device__ __forceinline__ int slabs() const {
-    const int64_t rem = npts - b * kTB;
-    const int64_t s = (rem + kTSlabN - 1) / kTSlabN;
-    return s < kTSlabs ? (int)s : kTSlabs;
+    const int s = (npts - b * kTB + kTSlabN - 1) / kTSlabN;
+    return s < kTSlabs ? s : kTSlabs;
   }
 };
 
@@ -339,7 +367,8 @@ __global__ void __launch_bounds__(kTThreads, 1)
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* sXb = reinterpret_cast<float*>(sm + Cfg::kOffXb);
-  double* sRow = reinterpret_cast<double*>(sm + Cfg::kOffRow);
+  float* sXa = reinterpret_cast<float*>(sm + Cfg::kOffXa);
+  float* sRow = reinterpret_cast<float*>(sm + Cfg::kOffRow);
   float* sCol = reinterpret_cast<float*>(sm + Cfg::kOffCol);
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + Cfg::kOffBar);
   uint64_t* a_full = bars + Cfg::kBarAFull;
@@ -361,8 +390,8 @@ __global__ void __launch_bounds__(kTThreads, 1)
     if (nact <= 0) return;
     const int64_t total = bm.act_ps[nact];
     const int64_t q = total / gridDim.x, rem = total % gridDim.x;
-    w0.p = c * q + (c < rem ? c : rem);
-    w0.p_end = w0.p + q + (c < rem ? 1 : 0);
+    w0.p = (int)(c * q + (c < rem ? c : rem));
+    w0.p_end = w0.p + (int)q + (c < rem ? 1 : 0);
     if (w0.p >= w0.p_end) return;
     int lo = 0, hi = nact - 1;
     while (lo < hi) {
@@ -371,8 +400,8 @@ __global__ void __launch_bounds__(kTThreads, 1)
     }
     w0.j = lo;
   } else {
-    w0.p = c * sp.q + (c < sp.rem ? c : sp.rem);
-    w0.p_end = w0.p + sp.q + (c < sp.rem ? 1 : 0);
+    w0.p = (int)(c * sp.q + (c < sp.rem ? c : sp.rem));
+    w0.p_end = w0.p + (int)sp.q + (c < sp.rem ? 1 : 0);
     if (w0.p >= w0.p_end) return;
   }
   w0.load_inst<BATCHED>(sp, bm, n);
@@ -394,7 +423,7 @@ __global__ void __launch_bounds__(kTThreads, 1)
     }
     for (int i = 0; i < kTBufs; ++i) {
       mbar_init(&acc_full[i], 1);
-      mbar_init(&acc_empty[i], kTEpi);
+      mbar_init(&acc_empty[i], kTEpi / 32);
     }
     mbar_init(drain, 1);
     *abort = 0;
@@ -405,28 +434,28 @@ __global__ void __launch_bounds__(kTThreads, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  int64_t b_issued = 0, a_issued = 0;  // copy role
+  uint32_t b_issued = 0, a_issued = 0;  // copy role
   bool mma_any = false;                // MMA role
   if (warp == kTCopyWarp) {
     // ---- copies ---------------------------------------------------------------
     if (lane == 0) {
       PairWalk wk = w0;
-      int64_t prev_a = -1;
+      int prev_a = -1;
       bool more = true;
       while (more && !*abort) {
-        const int64_t ab = wk.row_block();
+        const int ab = wk.row_block();
         if (ab != prev_a) {
-          if (!wait_or_abort(a_empty, (uint32_t)((a_issued & 1) ^ 1), status, abort)) break;
+          if (!wait_or_abort(a_empty, (a_issued & 1) ^ 1, status, abort)) break;
           mbar_arrive_expect_tx(a_full, Cfg::kHalf);
           bulk_g2s(sm + Cfg::kOffA, img + ab * (int64_t)kTImgBlock, Cfg::kHalf, a_full);
           ++a_issued;
           prev_a = ab;
         }
         const int bs = (int)(b_issued & 1);
-        if (!wait_or_abort(&b_empty[bs], (uint32_t)(((b_issued >> 1) & 1) ^ 1), status, abort)) break;
+        if (!wait_or_abort(&b_empty[bs], ((b_issued >> 1) & 1) ^ 1, status, abort)) break;
         mbar_arrive_expect_tx(&b_full[bs], Cfg::kHalf);
         bulk_g2s(sm + Cfg::kOffB + bs * Cfg::kHalf,
-                 img + wk.col_block() * (int64_t)kTImgBlock + Cfg::kHalf, Cfg::kHalf, &b_full[bs]);
+                 img + (int64_t)wk.col_block() * kTImgBlock + Cfg::kHalf, Cfg::kHalf, &b_full[bs]);
         ++b_issued;
         more = wk.next<BATCHED>(sp, bm, n);
       }
@@ -449,10 +478,11 @@ __global__ void __launch_bounds__(kTThreads, 1)
       constexpr uint64_t kStageStep = Cfg::kHalf >> 4;               // next column stage
       constexpr uint64_t kKStep = 32u >> 4;                          // TF32: second 8-wide K step
       PairWalk wk = w0;
-      int64_t prev_a = -1, na = 0, pc = 0, g = 0;
+      int prev_a = -1;
+      uint32_t na = 0, pc = 0, g = 0;
       bool more = true;
       while (more && !*abort) {
-        const int64_t ab = wk.row_block();
+        const int ab = wk.row_block();
         if (ab != prev_a) {
           if (!wait_or_abort(a_full, (uint32_t)(na & 1), status, abort)) break;
           ++na;
@@ -512,104 +542,105 @@ __global__ void __launch_bounds__(kTThreads, 1)
     // ---- epilogue (warps 0 .. 15) -------------------------------------------------
     const int q = warp & 3, cg = warp >> 2;
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
-    constexpr int XPT = kTB / kTEpi;  // x values of the column block per thread
+    static_assert(kTB == kTEpi, "one x value of each side per thread");
     PairWalk wk = w0;
-    int64_t pc = 0, g = 0;
-    bool dead = false;  // warp-uniform: stop waiting and reading TMEM after an abort
-    // x of the pair's column block (XPT per thread) and of this thread's rows,
-    // loaded one pair ahead
-    auto load_x = [&](const PairWalk& w, float (&xbv)[XPT], float (&xav)[kTRowTiles]) {
-#pragma unroll
-      for (int t = 0; t < XPT; ++t) {
-        const int64_t li = w.b * kTB + tid + t * kTEpi;
-        xbv[t] = li < w.npts ? x[w.seg + li] : 0.0f;
-      }
-#pragma unroll
-      for (int rt = 0; rt < kTRowTiles; ++rt) {
-        const int64_t li = w.a * kTB + rt * 128 + q * 32 + lane;
-        xav[rt] = li < w.npts ? x[w.seg + li] : 0.0f;
-      }
+    // warp-uniform: set when a wait gave up.  The warp then goes on without
+    // waiting, on whatever tensor memory holds (its sums are never used), so
+    // that its barrier arrivals still match the other warps'.
+    bool dead = wait_limit_ns() == 0;
+    if (dead) {
+      record_status(status, LAKER_ERR_TIMEOUT);
+      *abort = 1;
+    }
+    // x of a pair's column and row blocks into copy `set`
+    auto fetch_x = [&](const PairWalk& w, int set) {
+      const int lb = w.b * kTB + tid, la = w.a * kTB + tid;
+      const bool okb = lb < w.npts, oka = la < w.npts;
+      const float* pa = x + (oka ? w.seg + la : 0);
+      cp_async4(sXb + set * kTB + tid, x + (okb ? w.seg + lb : 0), okb);
+      cp_async4(sXa + 2 * (set * kTB + tid), pa, oka);
+      cp_async4(sXa + 2 * (set * kTB + tid) + 1, pa, oka);
     };
-    float xb_next[XPT], xa_next[kTRowTiles];
-    load_x(wk, xb_next, xa_next);
+    fetch_x(wk, 0);
+    // TMEM loads run one row tile ahead of the exponentials: `cur` holds the
+    // tile being consumed while the next one (of the next slab or pair too) is
+    // on its way into the other array.
+    uint32_t ra[16], rb[16];
+    constexpr int kUnits = kTRowTiles / UT;  // TMEM units per slab
+    const uint32_t tmem_me = tmem_base + lane_base + (uint32_t)(cg * CW);
+    uint32_t buf = 0, phase = 0;  // TMEM unit being read
+    // waits for the unit and issues the load of its first tile into r
+    auto open_unit = [&](uint32_t (&r)[16]) {
+      if (!__all_sync(0xffffffffu, dead || mbar_try_wait(&acc_full[buf], phase)))
+        dead = !warp_wait_or_abort(&acc_full[buf], phase, status, abort, lane);
+      tc_fence_after();
+      tmem_ld16_async(tmem_me + buf * (UT * kTSlabN), r);
+    };
+    cp_async_wait_all();
+    epi_bar_sync<kTEpi>();
+    open_unit(ra);
     bool more = true;
+    int pc = 0;
     while (more) {
       const int64_t slot = wk.slot();
       const bool off = wk.a != wk.b;
       const int nsl = wk.slabs();
-      float* xb = sXb + (pc & 1) * kTB;
+      const int xset = pc & 1, set = Cfg::kSets == 2 ? xset : 0;
+      more = wk.next<BATCHED>(sp, bm, n);
+      if (more) fetch_x(wk, xset ^ 1);
+      float2 xa[kTRowTiles];
 #pragma unroll
-      for (int t = 0; t < XPT; ++t) xb[tid + t * kTEpi] = xb_next[t];
-      float xa[kTRowTiles];
-#pragma unroll
-      for (int rt = 0; rt < kTRowTiles; ++rt) xa[rt] = xa_next[rt];
-      {
-        PairWalk nx = wk;
-        if (nx.next<BATCHED>(sp, bm, n)) load_x(nx, xb_next, xa_next);
-      }
-      epi_bar_sync<kTEpi>();
+      for (int rt = 0; rt < kTRowTiles; ++rt)
+        xa[rt] = reinterpret_cast<const float2*>(sXa)[xset * kTB + rt * 128 + q * 32 + lane];
       // a thread's share of a row sum (128 entries of the pair) in FP32, like
       // the column sums (512 rows per pair), widened to FP64 once per pair:
       // the per-chunk F2F + DADD chain cost 5 % of the kernel
       float racc[kTRowTiles];
 #pragma unroll
       for (int rt = 0; rt < kTRowTiles; ++rt) racc[rt] = 0.0f;
-      for (int s = 0; s < nsl; ++s) {
-        float xj[CW];
-        {
-          const float4* xs = reinterpret_cast<const float4*>(xb + s * kTSlabN + cg * CW);
+      const float4* xs = reinterpret_cast<const float4*>(sXb + xset * kTB + cg * CW);
+      float* cs_out = sCol + (set * 4 + q) * kTB + cg * CW + (lane >> 1);
+#pragma unroll 1
+      for (int s = nsl; s > 0; --s, xs += kTSlabN / 4, cs_out += kTSlabN) {
+        float2 xj[CW / 2];
 #pragma unroll
-          for (int u = 0; u < CW / 4; ++u) {
-            const float4 t = xs[u];
-            xj[4 * u] = t.x;
-            xj[4 * u + 1] = t.y;
-            xj[4 * u + 2] = t.z;
-            xj[4 * u + 3] = t.w;
-          }
+        for (int u = 0; u < CW / 4; ++u) {
+          const float4 t = xs[u];
+          xj[2 * u] = make_float2(t.x, t.y);
+          xj[2 * u + 1] = make_float2(t.z, t.w);
         }
         float2 cacc[CW / 2];
 #pragma unroll
-        for (int u = 0; u < CW / 2; ++u) cacc[u] = make_float2(0.0f, 0.0f);
-        // one tile's entries: exp2, row sum (packed pairs, fixed order) and
-        // column contributions (packed FFMA2: half the FMA-pipe instructions)
-        auto consume = [&](const float (&v)[CW], int rt) {
-          float2 ra = make_float2(0.0f, 0.0f);
-          const float2 xr = make_float2(xa[rt], xa[rt]);
+        for (int rt = 0; rt < kTRowTiles; ++rt) {
+          uint32_t(&cur)[16] = (rt & 1) ? rb : ra;
+          uint32_t(&nxt)[16] = (rt & 1) ? ra : rb;
+          tmem_ld_wait16(cur);
+          if (rt % UT == UT - 1) {
+            // the unit's last tile is in registers: release the buffer, go on
+            // to the next unit
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[buf]);
+            if (++buf == kTBufs) buf = 0, phase ^= 1;
+            if (rt / UT + 1 < kUnits || s > 1 || more) open_unit(nxt);
+          } else {
+            tmem_ld16_async(tmem_me + buf * (UT * kTSlabN) + (rt % UT + 1) * kTSlabN, nxt);
+          }
+          // the tile's entries: exp2, row sum (packed pairs, fixed order) and
+          // column contributions (packed FFMA2: half the FMA instructions)
+          float2 r2;
 #pragma unroll
           for (int u = 0; u < CW / 2; ++u) {
-            float2 e;
-            e.x = ex2_approx(CLAMP ? fminf(v[2 * u], kClampLog2) : v[2 * u]);
-            e.y = ex2_approx(CLAMP ? fminf(v[2 * u + 1], kClampLog2) : v[2 * u + 1]);
-            ra = __ffma2_rn(e, make_float2(xj[2 * u], xj[2 * u + 1]), ra);
-            cacc[u] = __ffma2_rn(e, xr, cacc[u]);
+            float2 e = make_float2(__uint_as_float(cur[2 * u]), __uint_as_float(cur[2 * u + 1]));
+            e.x = ex2_approx(CLAMP ? fminf(e.x, kClampLog2) : e.x);
+            e.y = ex2_approx(CLAMP ? fminf(e.y, kClampLog2) : e.y);
+            r2 = u == 0 ? __fmul2_rn(e, xj[u]) : __ffma2_rn(e, xj[u], r2);
+            cacc[u] = rt == 0 ? __fmul2_rn(e, xa[rt]) : __ffma2_rn(e, xa[rt], cacc[u]);
           }
-          racc[rt] += ra.x + ra.y;
-        };
-#pragma unroll
-        for (int hp = 0; hp < kTRowTiles / UT; ++hp, ++g) {
-          const int buf = (int)(g % kTBufs);
-          if (!dead)
-            dead = !warp_wait_or_abort(&acc_full[buf], (uint32_t)((g / kTBufs) & 1), status, abort, lane);
-          if (!dead) {
-            tc_fence_after();
-            const uint32_t t0 = tmem_base + lane_base + (uint32_t)(buf * (UT * kTSlabN) + cg * CW);
-            // tiles in pairs under one TMEM wait; the buffer is released after
-            // its last load, before the last pair is consumed
-#pragma unroll
-            for (int r2 = 0; r2 < UT; r2 += 2) {
-              float va[16], vb[16];
-              tmem_ld16x2(t0 + (uint32_t)(r2 * kTSlabN), t0 + (uint32_t)((r2 + 1) * kTSlabN), va, vb);
-              if (r2 + 2 == UT) {
-                tc_fence_before();
-                mbar_arrive(&acc_empty[buf]);
-              }
-              consume(va, UT * hp + r2);
-              consume(vb, UT * hp + r2 + 1);
-            }
-          }
+          racc[rt] += r2.x + r2.y;
         }
         if (off) {
-          // warp sums over its 4 x 32 rows; CW = 16: lanes 2c, 2c + 1 hold column c
+          // warp sums over its 4 x 32 rows; lanes 2c, 2c + 1 hold column c
           float cv[CW];
 #pragma unroll
           for (int u = 0; u < CW / 2; ++u) {
@@ -617,28 +648,31 @@ __global__ void __launch_bounds__(kTThreads, 1)
             cv[2 * u + 1] = cacc[u].y;
           }
           const float cs = warp_reduce_scatter<CW>(cv, lane);
-          if (CW == 32 || (lane & 1) == 0)
-            sCol[q * kTB + s * kTSlabN + cg * CW + (CW == 32 ? lane : (lane >> 1))] = cs;
+          if ((lane & 1) == 0) *cs_out = cs;
         }
       }
-      if (off && (CW == 32 || (lane & 1) == 0)) {
-        for (int s = nsl; s < kTSlabs; ++s)
-          sCol[q * kTB + s * kTSlabN + cg * CW + (CW == 32 ? lane : (lane >> 1))] = 0.0f;
+      if (off && (lane & 1) == 0) {
+        for (int s = nsl; s < kTSlabs; ++s, cs_out += kTSlabN) *cs_out = 0.0f;
       }
 #pragma unroll
-      for (int rt = 0; rt < kTRowTiles; ++rt) sRow[cg * kTB + rt * 128 + q * 32 + lane] = (double)racc[rt];
+      for (int rt = 0; rt < kTRowTiles; ++rt)
+        sRow[(set * kTNcg + cg) * kTB + rt * 128 + q * 32 + lane] = racc[rt];
+      cp_async_wait_all();
       epi_bar_sync<kTEpi>();
-      for (int j = tid; j < kTB; j += kTEpi) {
-        double r = sRow[j];
+      {
+        const float* rs = sRow + set * kTNcg * kTB + tid;
+        double r = (double)rs[0];
 #pragma unroll
-        for (int c = 1; c < kTNcg; ++c) r += sRow[c * kTB + j];
-        rowpart[slot * kTB + j] = r;
-        if (off)
-          colpart[slot * kTB + j] = ((sCol[j] + sCol[kTB + j]) + sCol[2 * kTB + j]) + sCol[3 * kTB + j];
+        for (int c = 1; c < kTNcg; ++c) r += (double)rs[c * kTB];
+        rowpart[slot * kTB + tid] = r;
+        const float* cp = sCol + set * 4 * kTB + tid;
+        if (off) colpart[slot * kTB + tid] = ((cp[0] + cp[kTB]) + cp[2 * kTB]) + cp[3 * kTB];
       }
+      if (Cfg::kSets == 1) epi_bar_sync<kTEpi>();  // one set: read before the next pair writes
       ++pc;
-      more = wk.next<BATCHED>(sp, bm, n);
     }
+    // after an abort the last load may still be on its way
+    tmem_ld_wait16(ra);
   }
 
   // ---- teardown: every role has left its loop ---------------------------------
@@ -647,7 +681,7 @@ __global__ void __launch_bounds__(kTThreads, 1)
     // bounded drains of the copies in flight and of the MMAs issued
     if (warp == kTCopyWarp && lane == 0) {
       if (a_issued > 0) mbar_wait_drain(a_full, (uint32_t)((a_issued - 1) & 1), status);
-      for (int64_t gg = b_issued > 2 ? b_issued - 2 : 0; gg < b_issued; ++gg)
+      for (uint32_t gg = b_issued > 2 ? b_issued - 2 : 0; gg < b_issued; ++gg)
         mbar_wait_drain(&b_full[gg & 1], (uint32_t)((gg >> 1) & 1), status);
     }
     if (warp == kTMmaWarp && lane == 0 && mma_any) {
@@ -668,6 +702,8 @@ cudaError_t launch_k1t_t(const uint8_t* img, int64_t n, const float* x, double* 
                          float* colpart, const SymPlan& sp, const BatchMap& bm, int* status,
                          const int* gate, cudaStream_t s) {
   using Cfg = K1tCfg<UT, FMT>;
+  // the walk's 32-bit pair and point numbers
+  if (sp.npairs >= (int64_t)1 << 31 || sp.nb * kTB >= (int64_t)1 << 31) return cudaErrorInvalidValue;
   static bool attr = false;
   if (!attr) {
     const cudaError_t e = cudaFuncSetAttribute(k1t_matvec<UT, FMT, CLAMP, BATCHED>,
