@@ -48,11 +48,13 @@ cudaError_t launch_k4(const double* rows64, int64_t m, const double* cols64, int
 cudaError_t launch_multi_f32(const float* rows32, int64_t m, const float* cols32, int64_t n, int d,
                              float lam, int clamp, const float* X, int k, int64_t ldx, float* Y,
                              int64_t ldy, cudaStream_t s, const int* gate = nullptr);
-// Y = B - (lam X + K X) when B != nullptr, else lam X + K X (FP64 throughout).
+// Y = B - (lam X + K X) when B != nullptr, else lam X + K X (FP64 throughout;
+// matvec_f64_multi.cu).  `part`: f64m_workspace_bytes(m, n, k) of scratch.
+size_t f64m_workspace_bytes(int64_t m, int64_t n, int k);
 cudaError_t launch_multi_f64(const double* rows64, int64_t m, const double* cols64, int64_t n, int d,
                              double lam, int clamp, const double* X, int k, int64_t ldx,
-                             const double* B, int64_t ldb, double* Y, int64_t ldy, cudaStream_t s,
-                             const int* gate = nullptr);
+                             const double* B, int64_t ldb, double* Y, int64_t ldy, double* part,
+                             cudaStream_t s, const int* gate = nullptr);
 
 // Tensor-core (tcgen05, split TF32) multi-RHS FP32 matvec (matvec_tc.cu).
 int k2_chunk_cols(int k);

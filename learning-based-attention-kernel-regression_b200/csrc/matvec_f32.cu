@@ -226,17 +226,15 @@ int k1_variant(int dp) {
 }
 
 // ---------------------------------------------------------------------------
-// Multi-RHS fused matvec on CUDA cores: Y = lam X + exp(Er Ec^T) X for
-// X (n x k).  A CTA owns a 64-row x 64-RHS output tile; per 32-column step it
-// evaluates the 64 x 32 block of kernel entries into shared memory (each
-// thread keeps one row embedding in registers) and multiplies it into X with
-// 4 x 4 register microtiles.  Row sums are flushed to FP64 every 256 columns.
-// Real = float: exp2 on MUFU with log2 e folded into the rows; Real = double:
-// FP64 logits and exp (the accurate operator, optionally as a residual).
-// Narrow products (k <= 16, e.g. the FP64 residual of a variance solve with
-// few queries) use 64 x 16 tiles of 64 threads instead, so that no
-// accumulation FMA lands on an absent right-hand side (LAKER_MULTI_NARROW=0
-// keeps the 64-wide tile for comparisons).
+// Multi-RHS fused FP32 matvec on CUDA cores (LAKER_K2_TC=0, for comparisons):
+// Y = lam X + exp(Er Ec^T) X for X (n x k).  A CTA owns a 64-row x 64-RHS
+// output tile; per 32-column step it evaluates the 64 x 32 block of kernel
+// entries into shared memory (each thread keeps one row embedding in registers,
+// log2 e folded in) and multiplies it into X with 4 x 4 register microtiles.
+// Row sums are flushed to FP64 every 256 columns.  Narrow products (k <= 16)
+// use 64 x 16 tiles of 64 threads instead, so that no accumulation FMA lands
+// on an absent right-hand side (LAKER_MULTI_NARROW=0 keeps the 64-wide tile for
+// comparisons).
 // ---------------------------------------------------------------------------
 constexpr int kMBM = 64, kMBN = 64, kMBK = 32, kMThreads = 256;
 constexpr int kMBNNarrow = 16;
@@ -252,63 +250,46 @@ bool multi_narrow_enabled() {
 
 }  // namespace
 
-template <typename Real, int DP, bool CLAMP, bool RESIDUAL, int BN = kMBN>
+template <int DP, bool CLAMP, int BN = kMBN>
 __global__ void __launch_bounds__((kMBM / 4) * (BN / 4))
-    multi_matvec_kernel(const Real* __restrict__ rows, int64_t m, const Real* __restrict__ cols,
-                        int64_t n, int col_layout_pairs, Real lam, const Real* __restrict__ X,
-                        int k, int64_t ldx, const Real* __restrict__ B, int64_t ldb,
-                        Real* __restrict__ Y, int64_t ldy, int row_layout_pairs,
-                        const int* gate) {
+    multi_matvec_kernel(const float* __restrict__ rows, int64_t m, const float* __restrict__ cols,
+                        int64_t n, float lam, const float* __restrict__ X, int k, int64_t ldx,
+                        float* __restrict__ Y, int64_t ldy, const int* gate) {
   if (gate && *gate == 0) return;
   constexpr int T = (kMBM / 4) * (BN / 4);  // threads: one 4 x 4 microtile each
   static_assert(T % kMBM == 0 && (kMBM * kMBK) % T == 0, "tile / thread mapping");
-  __shared__ __align__(16) Real sCol[kMBK][DP + 1];
-  __shared__ __align__(16) Real sP[kMBK][kMBM];
-  __shared__ __align__(16) Real sX[kMBK][BN];
-  __shared__ double sExp[64];
+  __shared__ __align__(16) float sCol[kMBK][DP + 1];
+  __shared__ __align__(16) float sP[kMBK][kMBM];
+  __shared__ __align__(16) float sX[kMBK][BN];
   const int tid = threadIdx.x;
-  if constexpr (sizeof(Real) == 8) exp_table_to_shared(sExp, tid, T);
   const int tx = tid % (BN / 4), ty = tid / (BN / 4);
   const int64_t i0 = (int64_t)blockIdx.x * kMBM;
   const int64_t c0 = (int64_t)blockIdx.y * BN;
 
-  auto emb = [&](const Real* base, int pairs, int64_t i, int kk) -> Real {
-    return pairs ? base[(i >> 1) * (DP * 2) + 2 * kk + (i & 1)] : base[i * DP + kk];
+  auto emb = [&](const float* base, int64_t i, int kk) -> float {
+    return base[(i >> 1) * (DP * 2) + 2 * kk + (i & 1)];
   };
 
   // The row this thread evaluates kernel entries for (fixed for the CTA).
   const int a = tid & (kMBM - 1);
-  Real rv[DP];
+  float rv[DP];
   {
     const int64_t i = i0 + a;
 #pragma unroll
-    for (int kk = 0; kk < DP; ++kk) {
-      Real v = (i < m) ? emb(rows, row_layout_pairs, i, kk) : Real(0);
-      if (sizeof(Real) == 4) v *= (Real)kLog2e;
-      rv[kk] = v;
-    }
+    for (int kk = 0; kk < DP; ++kk) rv[kk] = ((i < m) ? emb(rows, i, kk) : 0.0f) * kLog2e;
   }
-  // FP32: FP32 microtile sums flushed to FP64 every 8 steps; FP64: the
-  // microtile accumulates in FP64 directly
-  constexpr bool kF64 = sizeof(Real) == 8;
-  Real acc[4][4];
-  double acc64[kF64 ? 1 : 4][kF64 ? 1 : 4];
+  float acc[4][4];
+  double acc64[4][4];  // the microtile sums, flushed every 8 steps
 #pragma unroll
   for (int u = 0; u < 4; ++u)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) acc[u][v] = Real(0);
-  if constexpr (!kF64) {
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int v = 0; v < 4; ++v) acc64[u][v] = 0.0;
-  }
+    for (int v = 0; v < 4; ++v) acc[u][v] = 0.0f, acc64[u][v] = 0.0;
 
   // The next step's column embeddings and X tile are loaded into registers
   // while this step computes, and stored into shared memory after it.
   constexpr int kPC = (kMBK * DP + T - 1) / T, kPX = (kMBK * BN) / T;
   static_assert((kMBK * BN) % T == 0, "X tile / thread mapping");
-  Real pc[kPC], px[kPX];
+  float pc[kPC], px[kPX];
   auto fetch = [&](int st) {
     const int64_t j0 = (int64_t)st * kMBK;
 #pragma unroll
@@ -316,14 +297,14 @@ __global__ void __launch_bounds__((kMBM / 4) * (BN / 4))
       const int o = tid + t * T;
       const int jj = o / DP, kk = o - jj * DP;
       const int64_t j = j0 + jj;
-      pc[t] = (o < kMBK * DP && j < n) ? emb(cols, col_layout_pairs, j, kk) : Real(0);
+      pc[t] = (o < kMBK * DP && j < n) ? emb(cols, j, kk) : 0.0f;
     }
 #pragma unroll
     for (int t = 0; t < kPX; ++t) {
       const int o = tid + t * T;
       const int jj = o / BN, cc = o - jj * BN;
       const int64_t j = j0 + jj, c = c0 + cc;
-      px[t] = (j < n && c < k) ? X[j * ldx + c] : Real(0);
+      px[t] = (j < n && c < k) ? X[j * ldx + c] : 0.0f;
     }
   };
   auto store = [&]() {
@@ -350,23 +331,16 @@ __global__ void __launch_bounds__((kMBM / 4) * (BN / 4))
 #pragma unroll
     for (int q = 0; q < (kMBM * kMBK) / T; ++q) {
       const int jj = tid / kMBM + (T / kMBM) * q;
-      Real s = rv[0] * sCol[jj][0];
+      float s = rv[0] * sCol[jj][0];
 #pragma unroll
       for (int kk = 1; kk < DP; ++kk) s = fma(rv[kk], sCol[jj][kk], s);
-      Real e;
-      if constexpr (sizeof(Real) == 4) {
-        if (CLAMP) s = fminf(s, kClampLog2);
-        e = ex2_approx(s);
-      } else {
-        if (CLAMP) s = fmin(s, kClamp64);
-        e = exp_tab(s, sExp);
-      }
-      sP[jj][a] = e;
+      if (CLAMP) s = fminf(s, kClampLog2);
+      sP[jj][a] = ex2_approx(s);
     }
     __syncthreads();
 #pragma unroll 8
     for (int jj = 0; jj < kMBK; ++jj) {
-      Real pa[4], xb[4];
+      float pa[4], xb[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) pa[u] = sP[jj][ty * 4 + u], xb[u] = sX[jj][tx * 4 + u];
 #pragma unroll
@@ -374,13 +348,11 @@ __global__ void __launch_bounds__((kMBM / 4) * (BN / 4))
 #pragma unroll
         for (int v = 0; v < 4; ++v) acc[u][v] = fma(pa[u], xb[v], acc[u][v]);
     }
-    if constexpr (!kF64) {
-      if ((st & 7) == 7 || st == nsteps - 1) {
+    if ((st & 7) == 7 || st == nsteps - 1) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < 4; ++u)
 #pragma unroll
-          for (int v = 0; v < 4; ++v) acc64[u][v] += (double)acc[u][v], acc[u][v] = Real(0);
-      }
+        for (int v = 0; v < 4; ++v) acc64[u][v] += (double)acc[u][v], acc[u][v] = 0.0f;
     }
     __syncthreads();
     if (st + 1 < nsteps) store();
@@ -395,12 +367,9 @@ __global__ void __launch_bounds__((kMBM / 4) * (BN / 4))
     for (int v = 0; v < 4; ++v) {
       const int64_t c = c0 + tx * 4 + v;
       if (c >= k) continue;
-      double y;
-      if constexpr (kF64) y = acc[u][v];
-      else y = acc64[u][v];
+      double y = acc64[u][v];
       if (square) y += (double)lam * (double)X[i * ldx + c];
-      if (RESIDUAL) y = (double)B[i * ldb + c] - y;
-      Y[i * ldy + c] = (Real)y;
+      Y[i * ldy + c] = (float)y;
     }
   }
 }
@@ -413,40 +382,13 @@ cudaError_t launch_multi_f32_t(const float* rows, int64_t m, const float* cols, 
                                cudaStream_t s, const int* gate) {
   if (k <= kMBNNarrow && multi_narrow_enabled()) {
     dim3 grid((unsigned)ceil_div(m, kMBM), 1);
-    multi_matvec_kernel<float, DP, CLAMP, false, kMBNNarrow>
-        <<<grid, (kMBM / 4) * (kMBNNarrow / 4), 0, s>>>(rows, m, cols, n, 1, lam, X, k, ldx, nullptr,
-                                                        0, Y, ldy, 1, gate);
+    multi_matvec_kernel<DP, CLAMP, kMBNNarrow><<<grid, (kMBM / 4) * (kMBNNarrow / 4), 0, s>>>(
+        rows, m, cols, n, lam, X, k, ldx, Y, ldy, gate);
     return cudaGetLastError();
   }
   dim3 grid((unsigned)ceil_div(m, kMBM), (unsigned)ceil_div(k, kMBN));
-  multi_matvec_kernel<float, DP, CLAMP, false><<<grid, kMThreads, 0, s>>>(
-      rows, m, cols, n, 1, lam, X, k, ldx, nullptr, 0, Y, ldy, 1, gate);
-  return cudaGetLastError();
-}
-
-template <int DP, bool CLAMP>
-cudaError_t launch_multi_f64_t(const double* rows, int64_t m, const double* cols, int64_t n,
-                               double lam, const double* X, int k, int64_t ldx, const double* B,
-                               int64_t ldb, double* Y, int64_t ldy, cudaStream_t s,
-                               const int* gate) {
-  if (k <= kMBNNarrow && multi_narrow_enabled()) {
-    dim3 grid((unsigned)ceil_div(m, kMBM), 1);
-    constexpr int T = (kMBM / 4) * (kMBNNarrow / 4);
-    if (B)
-      multi_matvec_kernel<double, DP, CLAMP, true, kMBNNarrow><<<grid, T, 0, s>>>(
-          rows, m, cols, n, 0, lam, X, k, ldx, B, ldb, Y, ldy, 0, gate);
-    else
-      multi_matvec_kernel<double, DP, CLAMP, false, kMBNNarrow><<<grid, T, 0, s>>>(
-          rows, m, cols, n, 0, lam, X, k, ldx, nullptr, 0, Y, ldy, 0, gate);
-    return cudaGetLastError();
-  }
-  dim3 grid((unsigned)ceil_div(m, kMBM), (unsigned)ceil_div(k, kMBN));
-  if (B)
-    multi_matvec_kernel<double, DP, CLAMP, true><<<grid, kMThreads, 0, s>>>(
-        rows, m, cols, n, 0, lam, X, k, ldx, B, ldb, Y, ldy, 0, gate);
-  else
-    multi_matvec_kernel<double, DP, CLAMP, false><<<grid, kMThreads, 0, s>>>(
-        rows, m, cols, n, 0, lam, X, k, ldx, nullptr, 0, Y, ldy, 0, gate);
+  multi_matvec_kernel<DP, CLAMP>
+      <<<grid, kMThreads, 0, s>>>(rows, m, cols, n, lam, X, k, ldx, Y, ldy, gate);
   return cudaGetLastError();
 }
 
@@ -521,20 +463,6 @@ cudaError_t launch_multi_f32(const float* rows32, int64_t m, const float* cols32
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_multi_f64(const double* rows64, int64_t m, const double* cols64, int64_t n, int d,
-                             double lam, int clamp, const double* X, int k, int64_t ldx,
-                             const double* B, int64_t ldb, double* Y, int64_t ldy, cudaStream_t s,
-                             const int* gate) {
-  if (ceil_div(k, kMBN) > 65535) return cudaErrorInvalidValue;
-  const int dp = padded_dim(d);
-  if (clamp) {
-    LAKER_DISPATCH_DP(dp, return (launch_multi_f64_t<DPv, true>(rows64, m, cols64, n, lam, X, k, ldx, B, ldb, Y, ldy, s, gate)));
-  } else {
-    LAKER_DISPATCH_DP(dp, return (launch_multi_f64_t<DPv, false>(rows64, m, cols64, n, lam, X, k, ldx, B, ldb, Y, ldy, s, gate)));
-  }
-  return cudaErrorInvalidValue;
-}
-
 cudaError_t set_wait_limit_f32(unsigned long long ns) { return set_wait_limit_this_unit(ns); }
 
 cudaError_t launch_poison_on_status(const int* status, float* Y, int64_t m, int k, int64_t ldy,
@@ -552,6 +480,7 @@ using namespace laker;
 
 extern "C" size_t laker_matvec_workspace_bytes(int64_t m, int64_t n, int d, int k, int precision) {
   if (m < 0 || n < 0 || d < 1 || d > 16 || k < 1) return 0;
+  if (k > 1 && precision == 64) return kWsHeader + f64m_workspace_bytes(m, n, k);
   if (k > 1) {
     // the tensor-core paths stage X as split, swizzled TF32 tiles (and the
     // flash-style kernel the split-FP16 operand images of the points)

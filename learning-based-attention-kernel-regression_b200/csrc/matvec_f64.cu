@@ -217,7 +217,7 @@ extern "C" int laker_attn_matvec_f64(const double* rows64, int64_t m, const doub
   if (e != cudaSuccess) return fail_cuda(e);
   if (k > 1) {
     e = launch_multi_f64(rows64, m, cols64, n, d, (m == n) ? lam : 0.0, clamp, X, k, ldx, B, ldb,
-                         Y, ldy, s);
+                         Y, ldy, reinterpret_cast<double*>(static_cast<char*>(workspace) + kWsHeader), s);
     return e == cudaSuccess ? LAKER_OK : fail_cuda(e);
   }
   char* wbase = static_cast<char*>(workspace) + kWsHeader;

@@ -725,6 +725,7 @@ struct MpcgWs {
   float* AP;
   float* Z;
   double* bp;
+  double* part64;  // segment sums of the FP64 residual (may be empty)
   void* pscratch;
   uint8_t* img;
   size_t bytes;
@@ -768,6 +769,7 @@ MpcgWs carve_multi(void* base, int64_t n, int k, int nr) {
   w.AP = reinterpret_cast<float*>(take(nk * sizeof(float)));
   w.Z = reinterpret_cast<float*>(take(nk * sizeof(float)));
   w.bp = reinterpret_cast<double*>(take((size_t)3 * g.gx * (size_t)k * sizeof(double)));
+  w.part64 = reinterpret_cast<double*>(take(f64m_workspace_bytes(n, n, k)));
   w.pscratch = nr > 0 ? take(precond_multi_scratch_bytes(n, nr, k)) : nullptr;
   {
     // operator workspace: the tensor-core multi-RHS kernels' operand images
@@ -816,10 +818,10 @@ int pcg_solve_multi(const laker_operator* op, const laker_precond* pc, const dou
   // R = B - A64 X (gated by `gate`; ungated for the warm start)
   auto launch_residual = [&](int init, const int* gate, cudaStream_t cs) -> cudaError_t {
     cudaError_t ee = launch_multi_f64(op->packed64, n, op->packed64, n, d, op->lambda_reg, op->clamp,
-                                      X, k, k, B, k, w.R, k, cs, gate);
+                                      X, k, k, B, k, w.R, k, w.part64, cs, gate);
     if (ee == cudaSuccess)
       mp_after_residual_kernel<<<cgrid, kMT, 0, cs>>>(w.R, n, k, init, w.bp, w.st, w.cols);
-    launches += 2;
+    launches += f64m_workspace_bytes(n, n, k) > 0 ? 3 : 2;
     return ee;
   };
   auto launch_precond = [&](int init, cudaStream_t cs) -> cudaError_t {
