@@ -175,10 +175,10 @@ int laker_fp32_operator_kernel(int64_t n, int d);
 #define LAKER_VARIANT_WAIT_LIMIT_US 6
 /*   LAKER_VARIANT_MULTI_FLASH_K  multi-RHS FP32 products of unclamped
  *                                operators with at most this many right-hand
- *                                sides take the flash-style tensor-core kernel
- *                                (logits and P X on the tensor cores, P kept
- *                                in tensor memory; chunks of 32 right-hand
- *                                sides); 0 turns it off.  Default 32
+ *                                sides take the flash-style kernel (entries
+ *                                kept in registers between two warp-level
+ *                                tensor-core products; chunks of at most 64
+ *                                right-hand sides); 0 turns it off.  Default 96
  *                                (environment LAKER_MULTI_FLASH_K). */
 #define LAKER_VARIANT_MULTI_FLASH_K 7
 int laker_set_variant(int which, int value);

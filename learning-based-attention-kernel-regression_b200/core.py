@@ -240,7 +240,11 @@ class LAKERCore:
             kxq = ops.kernel_eval(op.packed.packed64, op.n, q64, end - start, d, not op.skip_clamp,
                                   True)
             v = pcg.solve(op.matvec, preconditioner.apply, kxq)
-            var[start:end] = ops.variance_finalize(q64, end - start, d, kxq, v)
+            # k^T A^-1 k = k^T v + v^T r + r^T A^-1 r with r = k - A v: the
+            # middle term makes the error quadratic in the solve's residual
+            # (first order, 1e-9 .. 1e-3 of sigma^2 at tol 1e-10 .. 1e-6)
+            r = op.residual_f64(v, kxq)
+            var[start:end] = ops.variance_finalize(q64, end - start, d, r.add_(kxq), v)
         _lib.raise_device_status(var.device)
         self.last_pcg = pcg
         return var.to(self.dtype)

@@ -46,10 +46,12 @@ int variant_default(int which) {
       const int v = atoi(e);
       if (v >= 0 && v <= 1 << 20) return v;
     }
-    // measured on B200 (n = 50k, k = 16: 3.73 vs 7.75 ms for the CUDA-core-
-    // logit kernel; n = 20k, k = 16: 0.70 vs 1.34 ms); wider products (one
-    // exp2 per entry per chunk of 32) are faster on the CUDA-core-logit kernel
-    return 32;
+    // Measured on B200 against the wide kernel (matvec_tc.cu), d = 10 / 16, us:
+    // n = 10,007: k = 48 192 / 197 vs 396 / 468, k = 64 239 / 246 vs 408 / 481,
+    // k = 96 338 / 349 vs 420 / 505, k = 128 426 / 438 vs 424 / 495;
+    // n = 40,000: k = 96 4450 / 4651 vs 4569 / 5653, k = 104 5674 / 5877 vs
+    // 3808 / 4886.
+    return 96;
   }
   const char* e = getenv("LAKER_K2_LOGITS_TC");
   return (e && e[0] == '1') ? 1 : 0;
