@@ -226,6 +226,101 @@ int k1_variant(int dp) {
 }
 
 // ---------------------------------------------------------------------------
+// Small square operators in one launch (k1d).  At n <= 3072 a product is a few
+// microseconds of arithmetic, and what the segment kernel spends is fill, partial
+// sums and a second launch.  Here every CTA copies all points into shared memory
+// (256-point tiles, one mbarrier each, so the first tile is used while the others
+// arrive), a warp takes R whole rows with its lanes over the column pairs, and the
+// row sum is finished in the warp: no partial sums, no finish kernel.  A lane adds
+// n / 64 pairs in FP32; lanes are added in FP64.
+// n = 1000: the product's C call 18.8 -> 8.2 us on the device (memset + segment
+// kernel + finish before, memset + this kernel now).
+// ---------------------------------------------------------------------------
+constexpr int kDWarps = 8, kDThreads = kDWarps * 32;
+constexpr int kDMaxTiles = 16;
+
+template <int DP, int R, bool CLAMP>
+__global__ void __launch_bounds__(kDThreads)
+    k1d_matvec_f32(const float* __restrict__ E, int64_t n, float lam, const float* __restrict__ x,
+                   float* __restrict__ y, int64_t ldy, int* status) {
+  constexpr int TC = kTileCols32;
+  constexpr uint32_t kTileBytes = TC * DP * 4;
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  const int ntiles = (int)ceil_div(n, TC);
+  float* sX = reinterpret_cast<float*>(sm + ntiles * kTileBytes);
+  __shared__ __align__(8) uint64_t bar[kDMaxTiles];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int t = 0; t < ntiles; ++t) mbar_init(&bar[t], 1);
+    mbar_fence_init();
+    for (int t = 0; t < ntiles; ++t) {
+      mbar_arrive_expect_tx(&bar[t], kTileBytes);
+      bulk_g2s(sm + t * kTileBytes, E + (int64_t)t * TC * DP, kTileBytes, &bar[t]);
+    }
+  }
+  for (int j = tid; j < ntiles * TC; j += kDThreads) sX[j] = j < n ? x[j] : 0.0f;
+  const int64_t i0 = ((int64_t)blockIdx.x * kDWarps + warp) * R;
+  float2 ev[R][DP];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int64_t i = i0 + r;
+    const float* blk = E + (i >> 1) * (DP * 2) + (i & 1);
+#pragma unroll
+    for (int k = 0; k < DP; ++k) {
+      const float v = i < n ? blk[2 * k] * kLog2e : 0.0f;
+      ev[r][k] = make_float2(v, v);
+    }
+  }
+  __syncthreads();
+  float2 acc[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) acc[r] = make_float2(0.0f, 0.0f);
+  bool ok = true;
+  for (int t = 0; t < ntiles; ++t) {
+    ok = ok && mbar_wait_bounded(&bar[t], 0u, status);
+    if (!ok) break;
+    const float* tile = reinterpret_cast<const float*>(sm + t * kTileBytes);
+    const float2* X2 = reinterpret_cast<const float2*>(sX + t * TC);
+#pragma unroll 2
+    for (int q = lane; q < TC / 2; q += 32) {
+      const float4* cp = reinterpret_cast<const float4*>(tile + q * (DP * 2));
+      float2 c[DP];
+#pragma unroll
+      for (int h = 0; h < DP / 2; ++h) {
+        const float4 v = cp[h];
+        c[2 * h] = make_float2(v.x, v.y);
+        c[2 * h + 1] = make_float2(v.z, v.w);
+      }
+      const float2 xv = X2[q];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float2 s = __fmul2_rn(ev[r][0], c[0]);
+#pragma unroll
+        for (int k = 1; k < DP; ++k) s = __ffma2_rn(ev[r][k], c[k], s);
+        if (CLAMP) {
+          s.x = fminf(s.x, kClampLog2);
+          s.y = fminf(s.y, kClampLog2);
+        }
+        acc[r] = __ffma2_rn(make_float2(ex2_approx(s.x), ex2_approx(s.y)), xv, acc[r]);
+      }
+    }
+  }
+  ok = __all_sync(0xffffffffu, ok);
+  if (!ok && tid == 0) {
+    // this CTA's copies must land before it exits
+    for (int t = 0; t < ntiles; ++t) mbar_wait_drain(&bar[t], 0u, status);
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const double v = warp_sum((double)acc[r].x + (double)acc[r].y);
+    const int64_t i = i0 + r;
+    if (lane == 0 && i < n)
+      y[i * ldy] = ok ? (float)fma((double)lam, (double)sX[i], v) : nan_f32();
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Multi-RHS fused FP32 matvec on CUDA cores (LAKER_K2_TC=0, for comparisons):
 // Y = lam X + exp(Er Ec^T) X for X (n x k).  A CTA owns a 64-row x 64-RHS
 // output tile; per 32-column step it evaluates the 64 x 32 block of kernel
@@ -429,6 +524,64 @@ __global__ void poison_on_status_kernel(const int* __restrict__ status, float* _
 
 }  // namespace
 
+namespace {
+
+size_t k1d_smem_bytes(int64_t n, int dp) {
+  return (size_t)ceil_div(n, kTileCols32) * (kTileCols32 * dp + kTileCols32) * 4 + 128;
+}
+
+// Rows per warp: the fewest that keep the grid within one CTA per SM (a CTA's
+// shared memory holds every point).
+int k1d_rows(int64_t n) {
+  const int64_t r = ceil_div(n, (int64_t)kDWarps * sm_count());
+  return r <= 1 ? 1 : r == 2 ? 2 : 3;
+}
+
+template <int DP, int R, bool CLAMP>
+cudaError_t launch_k1d_r(const float* E, int64_t n, float lam, const float* x, float* y, int64_t ldy,
+                         int* status, cudaStream_t s) {
+  static bool attr = false;
+  if (!attr) {
+    const cudaError_t e = cudaFuncSetAttribute(k1d_matvec_f32<DP, R, CLAMP>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+    if (e != cudaSuccess) return e;
+    attr = true;
+  }
+  k1d_matvec_f32<DP, R, CLAMP><<<(unsigned)ceil_div(n, kDWarps * R), kDThreads, k1d_smem_bytes(n, DP), s>>>(
+      E, n, lam, x, y, ldy, status);
+  return cudaGetLastError();
+}
+
+template <int DP, bool CLAMP>
+cudaError_t launch_k1d_t(const float* E, int64_t n, float lam, const float* x, float* y, int64_t ldy,
+                         int* status, cudaStream_t s) {
+  switch (k1d_rows(n)) {
+    case 1: return launch_k1d_r<DP, 1, CLAMP>(E, n, lam, x, y, ldy, status, s);
+    case 2: return launch_k1d_r<DP, 2, CLAMP>(E, n, lam, x, y, ldy, status, s);
+    default: return launch_k1d_r<DP, 3, CLAMP>(E, n, lam, x, y, ldy, status, s);
+  }
+}
+
+// Whether a square product takes k1d: every point fits a CTA's shared memory and
+// its 16 tiles (the symmetric kernels serve the larger operators).
+bool k1d_fits(int64_t n, int d) {
+  return n > 0 && n <= (int64_t)kDMaxTiles * kTileCols32 &&
+         k1d_smem_bytes(n, padded_dim(d)) <= 226 * 1024;
+}
+
+cudaError_t launch_k1d(const float* E, int64_t n, int d, float lam, int clamp, const float* x, float* y,
+                       int64_t ldy, int* status, cudaStream_t s) {
+  const int dp = padded_dim(d);
+  if (clamp) {
+    LAKER_DISPATCH_DP(dp, return (launch_k1d_t<DPv, true>(E, n, lam, x, y, ldy, status, s)));
+  } else {
+    LAKER_DISPATCH_DP(dp, return (launch_k1d_t<DPv, false>(E, n, lam, x, y, ldy, status, s)));
+  }
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace
+
 SegPlan k1_plan(int64_t m, int64_t n, int d) {
   const int dp = padded_dim(d);
   const int cfg = k1_variant(dp);
@@ -550,6 +703,10 @@ extern "C" int laker_attn_matvec_f32(const float* rows32, int64_t m, const float
     }
     if (e == cudaSuccess)
       e = launch_sym_finish(sp, rowpart, colpart, n, lam, X, Y, ldy, &hdr->status, s);
+    return e == cudaSuccess ? LAKER_OK : fail_cuda(e);
+  }
+  if (rows32 == cols32 && m == n && k1d_fits(n, d)) {
+    e = launch_k1d(cols32, n, d, lam, clamp, X, Y, ldy, &hdr->status, s);
     return e == cudaSuccess ? LAKER_OK : fail_cuda(e);
   }
   const SegPlan plan = k1_plan(m, n, d);
