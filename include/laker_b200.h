@@ -74,6 +74,12 @@ int laker_last_cuda_error(void);
  * breakdown). */
 int laker_workspace_status(const void* workspace, int* status, void* stream);
 
+/* Folds the status word of the last product that used `workspace` into the
+ * device word *sticky (the larger of the two), asynchronously on `stream`: a
+ * caller that launches many products reads one word later.  The products
+ * sharing a sticky word are on one stream. */
+int laker_workspace_status_fold(const void* workspace, int* sticky, void* stream);
+
 /* ------------------------------------------------------------------------ */
 /* Embedding layouts                                                         */
 /* ------------------------------------------------------------------------ */

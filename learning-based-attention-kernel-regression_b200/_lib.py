@@ -163,6 +163,7 @@ _SIGNATURES = {
     ),
     "laker_noalloc_status": (c_int, [POINTER(c_int), _P]),
     "laker_workspace_status": (c_int, [_P, POINTER(c_int), _P]),
+    "laker_workspace_status_fold": (c_int, [_P, _P, _P]),
     "laker_attn_matvec_f64": (
         c_int,
         [_P, c_int64, _P, c_int64, c_int, c_double, c_int, _P, c_int, c_int64, _P, c_int64, _P,
@@ -248,9 +249,15 @@ def check(status: int, where: str) -> None:
     raise LakerError(status, where, msg)
 
 
+# torch's current stream as a raw handle, without a Stream object per call
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream",
+                      lambda idx: torch.cuda.current_stream(idx).cuda_stream)
+
+
 def stream_handle(device: torch.device) -> int:
     """Raw cudaStream_t of torch's current stream on `device`."""
-    return torch.cuda.current_stream(device).cuda_stream
+    idx = device.index
+    return _raw_stream(idx if idx is not None else torch.cuda.current_device())
 
 
 def require_cuda(t: torch.Tensor, name: str) -> None:
@@ -277,15 +284,19 @@ def workspace(nbytes: int, device: torch.device) -> torch.Tensor:
 _pending_status: dict = {}
 
 
-def note_status(ws: torch.Tensor) -> None:
+def note_status(ws: torch.Tensor, stream: Optional[int] = None) -> None:
     """Fold the status word at the start of a product's workspace into the
     pending status of the current stream (asynchronous)."""
-    key = (ws.device.index, torch.cuda.current_stream(ws.device).cuda_stream)
+    device = ws.device
+    if stream is None:
+        stream = stream_handle(device)
+    key = (device.index, stream)
     acc = _pending_status.get(key)
     if acc is None:
-        acc = torch.zeros(1, dtype=torch.int32, device=ws.device)
+        acc = torch.zeros(1, dtype=torch.int32, device=device)
         _pending_status[key] = acc
-    torch.maximum(acc, ws[:4].view(torch.int32), out=acc)
+    check(load().laker_workspace_status_fold(ptr(ws), ptr(acc), stream),
+          "laker_workspace_status_fold")
 
 
 def raise_device_status(device: torch.device) -> None:
@@ -295,7 +306,7 @@ def raise_device_status(device: torch.device) -> None:
     if device.type != "cuda":
         return
     idx = device.index if device.index is not None else torch.cuda.current_device()
-    key = (idx, torch.cuda.current_stream(device).cuda_stream)
+    key = (idx, _raw_stream(idx))
     acc = _pending_status.get(key)
     if acc is None:
         return
@@ -362,13 +373,14 @@ def attn_matvec_f32(rows32, m, cols32, n, d, lam, clamp, X) -> torch.Tensor:
     k = 1 if X.dim() == 1 else X.shape[1]
     Y = torch.empty((m,) if X.dim() == 1 else (m, k), dtype=torch.float32, device=X.device)
     ws = workspace(lib.laker_matvec_workspace_bytes(m, n, d, k, 32), X.device)
+    stream = stream_handle(X.device)
     check(
         lib.laker_attn_matvec_f32(ptr(rows32), m, ptr(cols32), n, d, float(lam), int(clamp),
-                                  ptr(X), k, k, ptr(Y), k, ptr(ws), ws.numel(),
-                                  stream_handle(X.device)),
+                                  ptr(X), k, k, ptr(Y), k, ptr(ws), ws.numel(), stream),
         "laker_attn_matvec_f32",
     )
-    note_status(ws)
+    if m:  # without rows nothing ran and no status was written
+        note_status(ws, stream)
     return Y
 
 
@@ -380,13 +392,14 @@ def attn_matvec_f64(rows64, m, cols64, n, d, lam, clamp, X, B=None) -> torch.Ten
         B = B.contiguous()
     Y = torch.empty((m,) if X.dim() == 1 else (m, k), dtype=torch.float64, device=X.device)
     ws = workspace(lib.laker_matvec_workspace_bytes(m, n, d, k, 64), X.device)
+    stream = stream_handle(X.device)
     check(
         lib.laker_attn_matvec_f64(ptr(rows64), m, ptr(cols64), n, d, float(lam), int(clamp),
-                                  ptr(X), k, k, ptr(B), k, ptr(Y), k, ptr(ws), ws.numel(),
-                                  stream_handle(X.device)),
+                                  ptr(X), k, k, ptr(B), k, ptr(Y), k, ptr(ws), ws.numel(), stream),
         "laker_attn_matvec_f64",
     )
-    note_status(ws)
+    if k == 1 and m:  # the multi-RHS FP64 kernel has no bounded waits
+        note_status(ws, stream)
     return Y
 
 

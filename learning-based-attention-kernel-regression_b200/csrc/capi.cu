@@ -116,6 +116,11 @@ __global__ void __launch_bounds__(kPeakThreads) peak_dfma_kernel(int iters, doub
   if (s == 1234.5678) sink[0] = s;
 }
 
+__global__ void fold_status_kernel(const int* status, int* sticky) {
+  const int v = *status;
+  if (v > *sticky) *sticky = v;
+}
+
 template <typename F>
 int time_kernel(F launch, cudaStream_t s, float* ms_out) {
   cudaEvent_t e0, e1;
@@ -155,6 +160,14 @@ extern "C" int laker_workspace_status(const void* workspace, int* status, void* 
   if (e != cudaSuccess) return fail_cuda(e);
   *status = h;
   return LAKER_OK;
+}
+
+extern "C" int laker_workspace_status_fold(const void* workspace, int* sticky, void* stream) {
+  if (!workspace || !sticky) return LAKER_ERR_INVALID_ARG;
+  fold_status_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(
+      &static_cast<const WsHeader*>(workspace)->status, sticky);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? LAKER_OK : fail_cuda(e);
 }
 
 extern "C" const char* laker_status_string(int status) {

@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(T, 2)
         double s = ev[r][0] * c[0];
 #pragma unroll
         for (int k = 1; k < DP; ++k) s = fma(ev[r][k], c[k], s);
-        if (CLAMP) s = fmin(s, kClamp64);
+        if (CLAMP) s = s > kClamp64 ? kClamp64 : s;  // NaN stays NaN
         acc[r] = fma(exp_tab(s, sExp), xj, acc[r]);
       }
     }
@@ -149,6 +149,7 @@ __global__ void finish_f64_kernel(const double* __restrict__ part, int S, int64_
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m;
        i += (int64_t)gridDim.x * blockDim.x) {
     double acc = square ? lam * x[i * ldx] : 0.0;
+#pragma unroll 8
     for (int s = 0; s < S; ++s) acc += part[(int64_t)s * m + i];
     y[i * ldy] = failed ? nan_f64() : (b ? b[i * ldb] - acc : acc);
   }

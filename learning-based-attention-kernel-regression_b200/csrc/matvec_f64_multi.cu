@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kFmThreads, FmCfg<KS, NT, MT>::kMinCtas)
       for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-          p[mt][h] = exp_tab(CLAMP ? fmin(p[mt][h], kClamp64) : p[mt][h], sExp);
+          p[mt][h] = exp_tab(CLAMP && p[mt][h] > kClamp64 ? kClamp64 : p[mt][h], sExp);
 #pragma unroll
       for (int h = 0; h < 2; ++h)
 #pragma unroll

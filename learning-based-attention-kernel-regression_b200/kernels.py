@@ -99,15 +99,15 @@ class _AttnMatvec(torch.autograd.Function):
             X2 = x.detach().reshape(op.n, -1).to(op.dtype)
             G2 = gy.detach().reshape(op.n, -1).to(op.dtype)
             d = op.embedding_dim
-            gE = torch.zeros_like(E)
+            gE = None
             cols_per_chunk = max(1, 256 // (2 * d))  # right-hand sides per product
             for c0 in range(0, X2.shape[1], cols_per_chunk):
                 c1 = min(c0 + cols_per_chunk, X2.shape[1])
-                xs, gs = X2[:, c0:c1], G2[:, c0:c1]  # (n, c)
-                R = torch.cat([(xs.unsqueeze(2) * E.unsqueeze(1)).reshape(op.n, -1),
-                               (gs.unsqueeze(2) * E.unsqueeze(1)).reshape(op.n, -1)], dim=1)
-                KR = op._apply(R.contiguous(), 0.0).reshape(op.n, 2, c1 - c0, d)
-                gE += (gs.unsqueeze(2) * KR[:, 0]).sum(dim=1) + (xs.unsqueeze(2) * KR[:, 1]).sum(dim=1)
+                xg = torch.stack([X2[:, c0:c1], G2[:, c0:c1]], dim=1)  # (n, 2, c)
+                R = (xg.unsqueeze(3) * E.view(op.n, 1, 1, d)).reshape(op.n, -1)
+                KR = op._apply(R, 0.0).reshape(op.n, 2, c1 - c0, d)
+                part = (xg.flip(1).unsqueeze(3) * KR).sum(dim=(1, 2))
+                gE = part if gE is None else gE.add_(part)
             gE = gE.to(op.embeddings.dtype)
         return gE, gx, None
 
