@@ -156,6 +156,26 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
       : "memory");
 }
 
+// Stride (floats) of an embedding pair (2 DP floats) in shared memory that spreads
+// the 16-byte loads of lanes on consecutive pairs over all banks: 4 mod 8.
+__host__ __device__ constexpr int pair_stride(int dp) { return 2 * dp + (dp % 4 == 0 ? 4 : 0); }
+
+// Copies 16-byte chunks [0, pairs x DP / 2) of the packed pair layout at `src` into
+// pairs of pair_stride(DP) floats at `dst`, asynchronously by all T threads; the copies
+// complete a phase of `bar` (initialised with T arrivals).
+template <int DP, int T>
+__device__ __forceinline__ void stage_pairs(float* dst, const float* src, int pairs, uint64_t* bar,
+                                            int tid) {
+  constexpr int CH = DP / 2;
+  for (int e = tid; e < pairs * CH; e += T) {
+    const int q = e / CH, h = e - q * CH;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + q * pair_stride(DP) + 4 * h)),
+                 "l"(src + q * (2 * DP) + 4 * h)
+                 : "memory");
+  }
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(

@@ -86,6 +86,14 @@ cudaError_t launch_k2f(const float* rows32, int64_t m, const float* cols32, int6
                        float lam, const float* X, int64_t ldx, int k, float* Y, int64_t ldy,
                        uint8_t* ws, int* status, cudaStream_t s, const int* gate = nullptr);
 
+// ---- small single-RHS solves in one kernel (pcg_small.cu) ---------------------
+bool pcg_small_fits(int64_t n, int d, int nr, int ldq);
+size_t pcg_small_workspace_bytes(int64_t n, int nr);
+// -1: the grid cannot be resident at once here (nothing ran; take the other path)
+int pcg_solve_small(const laker_operator* op, const laker_precond* pc, const double* B, double* X,
+                    const laker_pcg_params* prm, void* workspace, laker_pcg_result* res,
+                    cudaStream_t s);
+
 // ---- multi-RHS solve and preconditioner apply (pcg_multi.cu) ----------------
 size_t pcg_multi_workspace_bytes(int64_t n, int d, int nr, int k);
 int pcg_solve_multi(const laker_operator* op, const laker_precond* pc, const double* B, int k,
@@ -108,6 +116,7 @@ cudaError_t set_wait_limit_sym(unsigned long long ns);
 cudaError_t set_wait_limit_symtc(unsigned long long ns);
 cudaError_t set_wait_limit_tc(unsigned long long ns);
 cudaError_t set_wait_limit_flash(unsigned long long ns);
+cudaError_t set_wait_limit_small(unsigned long long ns);
 
 // Y[i, c] = NaN for i < m, c < k when *status != 0: the outputs of a product
 // whose kernel recorded a device-side failure (a bounded wait that expired)

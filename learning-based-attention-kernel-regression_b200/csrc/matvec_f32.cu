@@ -230,7 +230,7 @@ int k1_variant(int dp) {
 // microseconds of arithmetic, and what the segment kernel spends is fill, partial
 // sums and a second launch.  Here every CTA copies all points into shared memory
 // (256-point tiles, one mbarrier each, so the first tile is used while the others
-// arrive), a warp takes R whole rows with its lanes over the column pairs, and the
+// arrive; pairs are spread so that no load has bank conflicts), a warp takes R whole rows with its lanes over the column pairs, and the
 // row sum is finished in the warp: no partial sums, no finish kernel.  A lane adds
 // n / 64 pairs in FP32; lanes are added in FP64.
 // n = 1000: the product's C call 18.8 -> 8.2 us on the device (memset + segment
@@ -243,22 +243,19 @@ template <int DP, int R, bool CLAMP>
 __global__ void __launch_bounds__(kDThreads)
     k1d_matvec_f32(const float* __restrict__ E, int64_t n, float lam, const float* __restrict__ x,
                    float* __restrict__ y, int64_t ldy, int* status) {
-  constexpr int TC = kTileCols32;
-  constexpr uint32_t kTileBytes = TC * DP * 4;
-  extern __shared__ __align__(128) uint8_t smem_raw[];
-  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  constexpr int TC = kTileCols32, PS = pair_stride(DP);
+  extern __shared__ __align__(128) float sm[];  // the pairs, then x
   const int ntiles = (int)ceil_div(n, TC);
-  float* sX = reinterpret_cast<float*>(sm + ntiles * kTileBytes);
+  float* sX = sm + ntiles * (TC / 2) * PS;
   __shared__ __align__(8) uint64_t bar[kDMaxTiles];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    for (int t = 0; t < ntiles; ++t) mbar_init(&bar[t], 1);
+    for (int t = 0; t < ntiles; ++t) mbar_init(&bar[t], kDThreads);
     mbar_fence_init();
-    for (int t = 0; t < ntiles; ++t) {
-      mbar_arrive_expect_tx(&bar[t], kTileBytes);
-      bulk_g2s(sm + t * kTileBytes, E + (int64_t)t * TC * DP, kTileBytes, &bar[t]);
-    }
   }
+  __syncthreads();
+  for (int t = 0; t < ntiles; ++t)
+    stage_pairs<DP, kDThreads>(sm + t * (TC / 2) * PS, E + (int64_t)t * TC * DP, TC / 2, &bar[t], tid);
   for (int j = tid; j < ntiles * TC; j += kDThreads) sX[j] = j < n ? x[j] : 0.0f;
   const int64_t i0 = ((int64_t)blockIdx.x * kDWarps + warp) * R;
   float2 ev[R][DP];
@@ -280,11 +277,11 @@ __global__ void __launch_bounds__(kDThreads)
   for (int t = 0; t < ntiles; ++t) {
     ok = ok && mbar_wait_bounded(&bar[t], 0u, status);
     if (!ok) break;
-    const float* tile = reinterpret_cast<const float*>(sm + t * kTileBytes);
+    const float* tile = sm + t * (TC / 2) * PS;
     const float2* X2 = reinterpret_cast<const float2*>(sX + t * TC);
 #pragma unroll 2
     for (int q = lane; q < TC / 2; q += 32) {
-      const float4* cp = reinterpret_cast<const float4*>(tile + q * (DP * 2));
+      const float4* cp = reinterpret_cast<const float4*>(tile + q * PS);
       float2 c[DP];
 #pragma unroll
       for (int h = 0; h < DP / 2; ++h) {
@@ -307,10 +304,8 @@ __global__ void __launch_bounds__(kDThreads)
     }
   }
   ok = __all_sync(0xffffffffu, ok);
-  if (!ok && tid == 0) {
-    // this CTA's copies must land before it exits
-    for (int t = 0; t < ntiles; ++t) mbar_wait_drain(&bar[t], 0u, status);
-  }
+  if (!ok)  // this thread's copies must land before it exits
+    asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const double v = warp_sum((double)acc[r].x + (double)acc[r].y);
@@ -527,7 +522,7 @@ __global__ void poison_on_status_kernel(const int* __restrict__ status, float* _
 namespace {
 
 size_t k1d_smem_bytes(int64_t n, int dp) {
-  return (size_t)ceil_div(n, kTileCols32) * (kTileCols32 * dp + kTileCols32) * 4 + 128;
+  return (size_t)ceil_div(n, kTileCols32) * (kTileCols32 / 2 * pair_stride(dp) + kTileCols32) * 4;
 }
 
 // Rows per warp: the fewest that keep the grid within one CTA per SM (a CTA's

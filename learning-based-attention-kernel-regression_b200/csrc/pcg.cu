@@ -419,7 +419,8 @@ using namespace laker;
 extern "C" size_t laker_pcg_workspace_bytes(int64_t n, int d, int nr, int k) {
   if (n < 1 || d < 1 || d > 16 || nr < 0 || nr > kMaxNr || k < 1) return 0;
   if (k != 1) return pcg_multi_workspace_bytes(n, d, nr, k);
-  return carve(nullptr, n, d, nr).bytes;
+  const size_t a = carve(nullptr, n, d, nr).bytes, b = pcg_small_workspace_bytes(n, nr);
+  return a > b ? a : b;
 }
 
 extern "C" int laker_pcg_solve(const laker_operator* op, const laker_precond* pc, const double* B,
@@ -437,6 +438,14 @@ extern "C" int laker_pcg_solve(const laker_operator* op, const laker_precond* pc
 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (k > 1) return pcg_solve_multi(op, pc, B, k, X, prm, workspace, res, s);
+  // Where the plain operator kernel would serve the iteration (n <= 3072 by default)
+  // and the operands fit on chip, the whole solve is one kernel; profiled solves
+  // (timed operator launches) and LAKER_PCG_GRAPH=0 keep separate launches.
+  if (prm->profile == 0 && pcg_use_graph() && !k1_symmetric_for(n) &&
+      pcg_small_fits(n, d, nr, pc ? pc->ldq : 0)) {
+    const int st = pcg_solve_small(op, pc, B, X, prm, workspace, res, s);
+    if (st >= 0) return st;
+  }
   PcgWs w = carve(workspace, n, d, nr);
   const SegPlan p1 = k1_plan(n, n, d), p4 = k4_plan(n, n, d);
   const bool sym = k1_symmetric_for(n);

@@ -72,7 +72,8 @@ cudaError_t apply_wait_limit(int us) {
   const unsigned long long ns = (unsigned long long)us * 1000ull;
   cudaError_t (*const setters[])(unsigned long long) = {set_wait_limit_f32, set_wait_limit_f64,
                                                         set_wait_limit_sym, set_wait_limit_symtc,
-                                                        set_wait_limit_tc, set_wait_limit_flash};
+                                                        set_wait_limit_tc, set_wait_limit_flash,
+                                                        set_wait_limit_small};
   for (auto f : setters) {
     const cudaError_t e = f(ns);
     if (e != cudaSuccess) return e;
