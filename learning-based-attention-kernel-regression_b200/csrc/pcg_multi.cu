@@ -193,6 +193,7 @@ __global__ void __launch_bounds__(kMT)
   const int c = blockIdx.y * kCW + threadIdx.x % kCW;
   double acc = 0.0;
   if (c < k) {
+#pragma unroll 4  // the loads of four rows in flight
     for (int64_t i = (int64_t)blockIdx.x * kRW + threadIdx.x / kCW; i < n;
          i += (int64_t)gridDim.x * kRW) {
       const int64_t e = i * k + c;
@@ -244,6 +245,7 @@ __global__ void __launch_bounds__(kMT)
   const int c = blockIdx.y * kCW + threadIdx.x % kCW;
   double d0 = 0.0, d1 = 0.0, d2 = 0.0;
   if (c < k) {
+#pragma unroll 4  // the loads of four rows in flight
     for (int64_t i = (int64_t)blockIdx.x * kRW + threadIdx.x / kCW; i < n;
          i += (int64_t)gridDim.x * kRW) {
       const double p = P[i * k + c], a = AP[i * k + c];
@@ -297,6 +299,7 @@ __global__ void __launch_bounds__(kMT)
   double acc = 0.0;
   if (c < k) {
     const double a = cols.alpha[c];
+#pragma unroll 4  // the loads of four rows in flight
     for (int64_t i = (int64_t)blockIdx.x * kRW + threadIdx.x / kCW; i < n;
          i += (int64_t)gridDim.x * kRW) {
       const int64_t e = i * k + c;
@@ -347,6 +350,7 @@ __global__ void __launch_bounds__(kMT)
   const int c = blockIdx.y * kCW + threadIdx.x % kCW;
   double acc = 0.0;
   if (c < k) {
+#pragma unroll 4  // the loads of four rows in flight
     for (int64_t i = (int64_t)blockIdx.x * kRW + threadIdx.x / kCW; i < n;
          i += (int64_t)gridDim.x * kRW) {
       const double r = R[i * k + c];
@@ -407,6 +411,7 @@ __global__ void __launch_bounds__(kMT)
   const int c = blockIdx.y * kCW + threadIdx.x % kCW;
   double acc = 0.0;
   if (c < k) {
+#pragma unroll 4  // the loads of four rows in flight
     for (int64_t i = (int64_t)blockIdx.x * kRW + threadIdx.x / kCW; i < n;
          i += (int64_t)gridDim.x * kRW) {
       const int64_t e = i * k + c;
@@ -456,6 +461,7 @@ __global__ void __launch_bounds__(kMT)
   if (c >= k) return;
   const bool live = cols.live[c] != 0;
   const float beta = (float)cols.beta[c];
+#pragma unroll 4  // the loads of four rows in flight
   for (int64_t i = (int64_t)blockIdx.x * kRW + threadIdx.x / kCW; i < n;
        i += (int64_t)gridDim.x * kRW) {
     const int64_t e = i * k + c;
@@ -467,10 +473,9 @@ __global__ void __launch_bounds__(kMT)
 
 // ---------------------------------------------------------------------------
 // Multi-RHS factored CCCP apply Z = c^-1/2 R + Q (W (Q^T R)), three tiled
-// CUDA-core GEMMs (64 x 64 output tiles, 4 x 4 register microtiles):
 //   project  U_chunk = Q[rows of the chunk]^T R[rows of the chunk]  (FP32
 //            products summed in FP32 within a row chunk, stored as FP64)
-//   core     V = W U with U = sum of the chunks in chunk order     (FP64)
+//   core     U = sum of the chunks in chunk order, V = W U          (FP64)
 //   expand   Z = c^-1/2 R + Q V                                      (FP32 sum)
 // It is only a preconditioner: FP32 sums change the iteration count, not the
 // accuracy of the solution, whose stop test is on the FP64 residual.  The
@@ -544,51 +549,55 @@ __global__ void __launch_bounds__(kMT)
   }
 }
 
+// U = sum of the projection's row chunks, in chunk order.
 __global__ void __launch_bounds__(kMT)
-    pcm_core_kernel(const float* __restrict__ W, int nr, int nq, const double* __restrict__ upart,
-                    int nchunk, int k, double* __restrict__ V, const int* gate) {
+    pcm_sum_kernel(const double* __restrict__ upart, int nchunk, int64_t total, double* __restrict__ U,
+                   const int* gate) {
   if (gate && *gate == 0) return;
-  __shared__ double Ws[kGK][kGT];
-  __shared__ double Us[kGK][kGT];
-  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-  const int j0 = blockIdx.x * kGT, c0 = blockIdx.y * kGT;
-  const int rr = tid / 16, cg = tid % 16;
-  double acc[4][4] = {};
-  for (int jp = 0; jp < nr; jp += kGK) {
-    const int jj = jp + rr;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int j = j0 + cg * 4 + v;
+  for (int64_t e = blockIdx.x * (int64_t)kMT + threadIdx.x; e < total; e += (int64_t)gridDim.x * kMT) {
+    double u = 0.0;
+#pragma unroll 8
+    for (int ch = 0; ch < nchunk; ++ch) u += upart[(int64_t)ch * total + e];
+    U[e] = u;
+  }
+}
+
+// V = W U (FP64).  The product is small (N_r^2 k FMAs) and was bound by latency: 64 x 64
+// tiles left 16 CTAs walking N_r with the chunk sums inside the loop (214 us at N_r =
+// 200, k = 256).  16 x 32 tiles give ~100 CTAs; a thread owns two outputs and adds the
+// N_r products in order, U and W staged 64 rows at a time.
+constexpr int kCoreJ = 16, kCoreC = 32, kCoreK = 64;
+__global__ void __launch_bounds__(kMT)
+    pcm_core_kernel(const float* __restrict__ W, int nr, int nq, const double* __restrict__ U, int k,
+                    double* __restrict__ V, const int* gate) {
+  if (gate && *gate == 0) return;
+  __shared__ double Ws[kCoreK][kCoreJ];
+  __shared__ double Us[kCoreK][kCoreC];
+  const int tid = threadIdx.x, c = tid % kCoreC, j = tid / kCoreC;  // outputs (j, c), (j + 8, c)
+  const int j0 = blockIdx.x * kCoreJ, c0 = blockIdx.y * kCoreC;
+  double a0 = 0.0, a1 = 0.0;
+  for (int jp = 0; jp < nr; jp += kCoreK) {
+    for (int e = tid; e < kCoreK * kCoreJ; e += kMT) {
+      const int r = e / kCoreJ, q = e % kCoreJ;
       // W is symmetric: W[j][jj] = W[jj][j] (row jj read contiguously)
-      Ws[rr][cg * 4 + v] = (jj < nr && j < nr) ? (double)W[(int64_t)jj * nr + j] : 0.0;
-      const int c = c0 + cg * 4 + v;
-      double u = 0.0;
-      if (jj < nr && c < k)
-        for (int ch = 0; ch < nchunk; ++ch) u += upart[((int64_t)ch * nq + jj) * k + c];
-      Us[rr][cg * 4 + v] = u;
+      Ws[r][q] = (jp + r < nr && j0 + q < nr) ? (double)W[(int64_t)(jp + r) * nr + j0 + q] : 0.0;
+    }
+    for (int e = tid; e < kCoreK * kCoreC; e += kMT) {
+      const int r = e / kCoreC, q = e % kCoreC;
+      Us[r][q] = (jp + r < nr && c0 + q < k) ? U[(int64_t)(jp + r) * k + c0 + q] : 0.0;
     }
     __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kGK; ++kk) {
-      double av[4], bv[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) av[u] = Ws[kk][ty * 4 + u], bv[u] = Us[kk][tx * 4 + u];
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = fma(av[u], bv[v], acc[u][v]);
+#pragma unroll 16
+    for (int r = 0; r < kCoreK; ++r) {
+      const double u = Us[r][c];
+      a0 = fma(Ws[r][j], u, a0);
+      a1 = fma(Ws[r][j + 8], u, a1);
     }
     __syncthreads();
   }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int j = j0 + ty * 4 + u;
-    if (j >= nq) continue;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int c = c0 + tx * 4 + v;
-      if (c < k) V[(int64_t)j * k + c] = acc[u][v];
-    }
+  if (c0 + c < k) {
+    if (j0 + j < nq) V[(int64_t)(j0 + j) * k + c0 + c] = a0;
+    if (j0 + j + 8 < nq) V[(int64_t)(j0 + j + 8) * k + c0 + c] = a1;
   }
 }
 
@@ -683,7 +692,7 @@ size_t precond_multi_scratch_bytes(int64_t n, int nr, int k) {
   const int nq = pcm_cols(nr);
   const int nch = pcm_chunks(n, nq, k);
   return (size_t)round_up((int64_t)((size_t)nch * nq * k * sizeof(double)), 256) +
-         (size_t)round_up((int64_t)((size_t)nq * k * sizeof(double)), 256);
+         2 * (size_t)round_up((int64_t)((size_t)nq * k * sizeof(double)), 256);
 }
 
 template <typename ZT>
@@ -699,8 +708,11 @@ cudaError_t launch_precond_multi(const laker_precond* pc, const double* R, int k
   const unsigned gy = (unsigned)ceil_div(k, kGT);
   pcm_project_kernel<<<dim3((unsigned)ceil_div(nq, kGT), gy, (unsigned)nch), kMT, 0, s>>>(
       pc->q_basis, ldq, nq, R, n, k, chunk_rows, upart, gate);
-  pcm_core_kernel<<<dim3((unsigned)ceil_div(nq, kGT), gy), kMT, 0, s>>>(pc->w_core, nr, nq, upart,
-                                                                      nch, k, V, gate);
+  double* U = V + round_up((int64_t)nq * k, 32);
+  const int64_t total = (int64_t)nq * k;
+  pcm_sum_kernel<<<(unsigned)ceil_div(total, kMT), kMT, 0, s>>>(upart, nch, total, U, gate);
+  pcm_core_kernel<<<dim3((unsigned)ceil_div(nq, kCoreJ), (unsigned)ceil_div(k, kCoreC)), kMT, 0, s>>>(
+      pc->w_core, nr, nq, U, k, V, gate);
   pcm_expand_kernel<ZT><<<dim3((unsigned)ceil_div(n, kGT), gy), kMT, 0, s>>>(
       pc->q_basis, ldq, nq, nr, V, R, pc->inv_sqrt_iso, n, k, Z, gate);
   return cudaGetLastError();
@@ -829,7 +841,7 @@ int pcg_solve_multi(const laker_operator* op, const laker_precond* pc, const dou
     if (pc) {
       ee = launch_precond_multi<float>(pc, w.R, k, w.Z, w.pscratch, &w.st->active, cs);
       mp_after_precond_kernel<false><<<cgrid, kMT, 0, cs>>>(w.R, w.Z, n, k, init, w.bp, w.st, w.cols);
-      launches += 4;
+      launches += 5;
     } else {
       mp_after_precond_kernel<true><<<cgrid, kMT, 0, cs>>>(w.R, w.Z, n, k, init, w.bp, w.st, w.cols);
       launches += 1;
