@@ -65,12 +65,6 @@ cudaError_t launch_k2(const float* rows32, int64_t m, const float* cols32, int64
                       int64_t ldy, uint8_t* img, int* status, cudaStream_t s,
                       const int* gate = nullptr);
 
-// Split, swizzled TF32 image of X (n x k) in 32-point tiles of N right-hand
-// sides (the multi-RHS kernels' B operand): chunk c, tile t at
-// (c * ntiles + t) * N * 256 bytes, [hi: N rows x 128 B][lo: N rows x 128 B]
-// in the 128-byte-swizzled K-major layout; points past n are zero.
-cudaError_t launch_pack_x32(const float* X, int64_t n, int64_t ldx, int k, int N, int64_t ntiles,
-                            uint8_t* img, const int* gate, cudaStream_t s);
 // Y = lam X + sum over `segs` segment partials (segs x m x k floats), in
 // segment order.
 cudaError_t launch_seg_reduce(const float* part, int segs, int64_t m, int k, float lam,

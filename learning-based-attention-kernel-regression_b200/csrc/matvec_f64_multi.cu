@@ -178,18 +178,25 @@ __global__ void __launch_bounds__(kFmThreads, FmCfg<KS, NT, MT>::kMinCtas)
     if (i >= m) continue;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
+    {
+      const int c = c0 + nt * 8 + 2 * t;
+      if (part && (k & 1) == 0 && c < k) {  // both columns, 16-byte aligned
+        *reinterpret_cast<double2*>(part + ((int64_t)blockIdx.z * m + i) * k + c) =
+            make_double2(acc[mt][nt][0], acc[mt][nt][1]);
+        continue;
+      }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int c = c0 + nt * 8 + 2 * t + h;
-        if (c >= k) continue;
+        if (c + h >= k) continue;
         double y = acc[mt][nt][h];
         if (part) {
-          part[((int64_t)blockIdx.z * m + i) * k + c] = y;
+          part[((int64_t)blockIdx.z * m + i) * k + c + h] = y;
         } else {
-          if (square) y = fma(lam, X[i * ldx + c], y);
-          Y[i * ldy + c] = B ? B[i * ldb + c] - y : y;
+          if (square) y = fma(lam, X[i * ldx + c + h], y);
+          Y[i * ldy + c + h] = B ? B[i * ldb + c + h] - y : y;
         }
       }
+    }
   }
 }
 
@@ -205,6 +212,7 @@ __global__ void f64m_reduce_kernel(const double* __restrict__ part, int S, int64
     const int64_t i = e / k;
     const int c = (int)(e - i * k);
     double y = 0.0;
+#pragma unroll 4  // loads in flight, added in segment order
     for (int s = 0; s < S; ++s) y += part[(int64_t)s * total + e];
     if (square) y = fma(lam, X[i * ldx + c], y);
     Y[i * ldy + c] = B ? B[i * ldb + c] - y : y;

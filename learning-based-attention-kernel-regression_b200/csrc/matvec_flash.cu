@@ -275,12 +275,24 @@ __global__ void __launch_bounds__(kFThreads, 2)
 #pragma unroll
     for (int q = 0; q < NT; ++q)
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int64_t row = row0 + 16 * i + g + 8 * (u >> 1);
-        const int col = blockIdx.y * (NT * 8) + q * 8 + 2 * t + (u & 1);
+      for (int h = 0; h < 2; ++h) {
+        const int64_t row = row0 + 16 * i + g + 8 * h;
+        const int col = blockIdx.y * (NT * 8) + q * 8 + 2 * t;  // and col + 1
         if (row >= m || col >= k) continue;
-        if (part) part[((int64_t)blockIdx.z * m + row) * k + col] = sum[i][q][u];
-        else Y[row * ldy + col] = lam != 0.0f ? fmaf(lam, X[row * ldx + col], sum[i][q][u]) : sum[i][q][u];
+        const float v0 = sum[i][q][2 * h], v1 = sum[i][q][2 * h + 1];
+        if (part) {
+          float* dst = part + ((int64_t)blockIdx.z * m + row) * k + col;
+          if ((k & 1) == 0) {  // 8-byte aligned, and col + 1 < k
+            *reinterpret_cast<float2*>(dst) = make_float2(v0, v1);
+          } else {
+            dst[0] = v0;
+            if (col + 1 < k) dst[1] = v1;
+          }
+        } else {
+          Y[row * ldy + col] = lam != 0.0f ? fmaf(lam, X[row * ldx + col], v0) : v0;
+          if (col + 1 < k)
+            Y[row * ldy + col + 1] = lam != 0.0f ? fmaf(lam, X[row * ldx + col + 1], v1) : v1;
+        }
       }
 }
 

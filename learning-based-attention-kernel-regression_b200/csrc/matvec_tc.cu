@@ -74,23 +74,30 @@ template <int TK>
 __global__ void k2_pack_x(const float* __restrict__ X, int64_t n, int64_t ldx, int k, int N,
                           int64_t ntiles, uint8_t* __restrict__ img, const int* gate) {
   if (gate && *gate == 0) return;
-  constexpr int kTcTileK = TK;
-  const int64_t total = (int64_t)ntiles * kTcTileK * ((k + N - 1) / N) * N;
+  // e enumerates (four points 4 j4 .. + 3, padded rhs q) with q fastest: coalesced reads
+  // of X, one 16-byte store per part
+  const int kp = ((k + N - 1) / N) * N;
+  const int64_t total = ntiles * (TK / 4) * kp;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
        e += (int64_t)gridDim.x * blockDim.x) {
-    // e enumerates (point j, padded rhs q) with q fastest: coalesced reads of X
-    const int kp = ((k + N - 1) / N) * N;
-    const int64_t j = e / kp;
-    const int q = (int)(e - j * kp);
-    const float v = (j < n && q < k) ? X[j * ldx + q] : 0.0f;
-    const uint32_t hi = to_tf32(v);
-    const uint32_t lo = to_tf32(v - __uint_as_float(hi));
-    const int64_t c = q / N, t = j / kTcTileK;
-    const int r = q - (int)c * N, kk = (int)(j - t * kTcTileK);
+    const int64_t j4 = e / kp;
+    const int q = (int)(e - j4 * kp);
+    uint4 hi, lo;
+    uint32_t* ph = &hi.x;
+    uint32_t* pl = &lo.x;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t j = 4 * j4 + u;
+      const float v = (j < n && q < k) ? X[j * ldx + q] : 0.0f;
+      ph[u] = to_tf32(v);
+      pl[u] = to_tf32(v - __uint_as_float(ph[u]));
+    }
+    const int64_t c = q / N, t = j4 / (TK / 4);
+    const int r = q - (int)c * N, kk = (int)(4 * (j4 - t * (TK / 4)));
     uint8_t* blk = img + ((c * ntiles + t) * (int64_t)N * (8 * TK));
     const uint32_t off = TileCfg<TK>::offset((uint32_t)r, (uint32_t)kk);
-    *reinterpret_cast<uint32_t*>(blk + off) = hi;
-    *reinterpret_cast<uint32_t*>(blk + (int64_t)N * (4 * TK) + off) = lo;
+    *reinterpret_cast<uint4*>(blk + off) = hi;
+    *reinterpret_cast<uint4*>(blk + (int64_t)N * (4 * TK) + off) = lo;
   }
 }
 
@@ -99,22 +106,29 @@ __global__ void k2_pack_x(const float* __restrict__ X, int64_t n, int64_t ldx, i
 // persistent grid takes items round-robin, so every SM stays busy whatever
 // the number of row tiles.  Roles inside a CTA (no CTA-wide barrier in the
 // main loop; full/empty mbarrier rings between the roles):
-//   warps 0-7  entries: per tile, wait for the column embeddings, wait for a
+//   warps 0-15 entries: per tile, wait for the column embeddings, wait for a
 //              free A slot, write the TK x 128 entries as split TF32 into it,
 //              arrive on its "full" barrier; per item, after the last tile,
 //              wait for the accumulators, read them from TMEM and write the
 //              item's output (Y, or a segment partial), free the TMEM buffer
-//   warp 8     copies: per tile, wait for a free B stage, TMA the X image
+//   warp 16    copies: per tile, wait for a free B stage, TMA the X image
 //              slice and the column embeddings into it
-//   warp 9     MMA: per tile, wait for A and B, issue the three split-TF32
+//   warp 17    MMA: per tile, wait for A and B, issue the three split-TF32
 //              products per 8-point K step, commit to the A slot's and the B
 //              stage's "empty" barriers; per item, commit to the TMEM
 //              buffer's "full" barrier (two TMEM buffers: the epilogue of one
 //              item overlaps the MMAs of the next)
 // Every wait is bounded; a timeout raises a shared abort flag that every role
 // checks, then the CTA drains its copies and MMAs and frees TMEM.
-constexpr int kEntryThreads = 256;
+// 16 entry warps, four threads per row: with 8 the entries' latency (broadcast loads,
+// ex2, the split) showed between the MMAs.  The larger loss was the epilogue's
+// 4-byte stores at a stride of k floats; 16-byte stores of the segment sums took
+// n = 10,000, k = 512 from 878 to 684 us (932 with 8 warps), n = 20,000, k = 256 from
+// 1391 to 1213 us (1453), n = 40,000, k = 256 4464 us (4697): 0.54, 0.61 and 0.67 of the
+// TF32 rate (half the measured bf16 burst), the same bits.
+constexpr int kEntryThreads = 512;
 constexpr int kTcThreadsWs = kEntryThreads + 64;  // + copy warp + MMA warp
+constexpr int kTcCopyWarp = kEntryThreads / 32, kTcMmaWarp = kTcCopyWarp + 1;
 constexpr int kASlots = 2;
 
 struct K2Work {
@@ -194,7 +208,7 @@ __global__ void __launch_bounds__(kTcThreadsWs, 1)
 
   int64_t b_issued = 0;     // copy role: tiles issued
   int64_t mma_tiles = 0;
-  if (warp == 8) {
+  if (warp == kTcCopyWarp) {
     // ---- copies ------------------------------------------------------------
     if (lane == 0) {
       int64_t g = 0;  // tile counter over this CTA's items
@@ -213,7 +227,7 @@ __global__ void __launch_bounds__(kTcThreadsWs, 1)
       }
       b_issued = g;
     }
-  } else if (warp == 9) {
+  } else if (warp == kTcMmaWarp) {
     // ---- MMA issue -----------------------------------------------------------
     if (lane == 0) {
       int64_t g = 0, ni = 0;
@@ -254,8 +268,8 @@ __global__ void __launch_bounds__(kTcThreadsWs, 1)
       mma_tiles = g;
     }
   } else {
-    // ---- entries + epilogue (warps 0-7) ------------------------------------
-    const int row = tid & 127, half = tid >> 7;
+    // ---- entries + epilogue (warps 0-15) -----------------------------------
+    const int row = tid & 127, part4 = tid >> 7;  // four threads per row
     int64_t g = 0, ni = 0;
     // waits are made warp-uniform (__all_sync) so that a warp reaches the
     // .sync.aligned TMEM loads with all its lanes or not at all
@@ -288,15 +302,21 @@ __global__ void __launch_bounds__(kTcThreadsWs, 1)
         uint8_t* a_hi = sA + as * 2 * kABytes;
         uint8_t* a_lo = a_hi + kABytes;
 #pragma unroll
-        for (int cc = 0; cc < TK / 8; ++cc) {
-          const int c = (TK / 8) * half + cc;  // 16-byte chunk: points 4c .. 4c+3
+        for (int cc = 0; cc < TK / 16; ++cc) {
+          const int c = (TK / 16) * part4 + cc;  // 16-byte chunk: points 4c .. 4c+3
           float p[4];
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const float* pe = ec + (2 * c + h) * (DP * 2);
-            float2 sacc = __fmul2_rn(ev[0], make_float2(pe[0], pe[1]));
+            // a point pair's embeddings, DP / 2 broadcast loads
+            const float4* pe = reinterpret_cast<const float4*>(ec + (2 * c + h) * (DP * 2));
+            float2 sacc;
 #pragma unroll
-            for (int q = 1; q < DP; ++q) sacc = __ffma2_rn(ev[q], make_float2(pe[2 * q], pe[2 * q + 1]), sacc);
+            for (int q = 0; q < DP / 2; ++q) {
+              const float4 e4 = pe[q];
+              sacc = q == 0 ? __fmul2_rn(ev[0], make_float2(e4.x, e4.y))
+                            : __ffma2_rn(ev[2 * q], make_float2(e4.x, e4.y), sacc);
+              sacc = __ffma2_rn(ev[2 * q + 1], make_float2(e4.z, e4.w), sacc);
+            }
             if (CLAMP) {
               sacc.x = fminf(sacc.x, kClampLog2);
               sacc.y = fminf(sacc.y, kClampLog2);
@@ -306,15 +326,15 @@ __global__ void __launch_bounds__(kTcThreadsWs, 1)
           }
           uint4 hi, lo;
           // P_hi by truncation (an AND), P_lo the exact remainder rounded to
-          // TF32: |error| <= 2^-22 |p|
+          // TF32 (half a unit added, then truncated): |error| <= 2^-22 |p|
           hi.x = __float_as_uint(p[0]) & 0xffffe000u;
           hi.y = __float_as_uint(p[1]) & 0xffffe000u;
           hi.z = __float_as_uint(p[2]) & 0xffffe000u;
           hi.w = __float_as_uint(p[3]) & 0xffffe000u;
-          lo.x = to_tf32(p[0] - __uint_as_float(hi.x));
-          lo.y = to_tf32(p[1] - __uint_as_float(hi.y));
-          lo.z = to_tf32(p[2] - __uint_as_float(hi.z));
-          lo.w = to_tf32(p[3] - __uint_as_float(hi.w));
+          lo.x = (__float_as_uint(p[0] - __uint_as_float(hi.x)) + 0x1000u) & 0xffffe000u;
+          lo.y = (__float_as_uint(p[1] - __uint_as_float(hi.y)) + 0x1000u) & 0xffffe000u;
+          lo.z = (__float_as_uint(p[2] - __uint_as_float(hi.z)) + 0x1000u) & 0xffffe000u;
+          lo.w = (__float_as_uint(p[3] - __uint_as_float(hi.w)) + 0x1000u) & 0xffffe000u;
           const uint32_t off = TileCfg<TK>::offset((uint32_t)row, (uint32_t)(4 * c));
           *reinterpret_cast<uint4*>(a_hi + off) = hi;
           *reinterpret_cast<uint4*>(a_lo + off) = lo;
@@ -331,12 +351,18 @@ __global__ void __launch_bounds__(kTcThreadsWs, 1)
       tc_fence_after();
       const int64_t r = rt * kTcRows + (warp & 3) * 32 + lane;
       const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-      const int nh = N / 2, c_begin = (warp >> 2) * nh;
       const int sg = (int)(t0 / wk.tps);
-      for (int c0 = c_begin; c0 < c_begin + nh; c0 += 16) {
+      for (int c0 = (warp >> 2) * 16; c0 < N; c0 += 64) {
         float v[16];
         tmem_ld16(tmem_base + (uint32_t)(ab * 256) + lane_base + (uint32_t)c0, v);
-        if (r < m) {
+        if (r < m && wk.segs > 1 && (k & 3) == 0 && ch * N + c0 + 16 <= k) {
+          // whole 16-byte chunks of the segment's partial sums (1 KB aligned):
+          // a quarter of the store instructions
+          float4* dst = reinterpret_cast<float4*>(part + ((int64_t)sg * m + r) * k + ch * N + c0);
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            dst[u] = make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+        } else if (r < m) {
 #pragma unroll
           for (int u = 0; u < 16; ++u) {
             const int q = ch * N + c0 + u;
@@ -360,13 +386,13 @@ __global__ void __launch_bounds__(kTcThreadsWs, 1)
   if (*abort) {
     // bounded drains: the copies the copy role issued and the MMAs the MMA
     // role committed (the last commit of each barrier covers earlier ones)
-    if (warp == 8 && lane == 0) {
+    if (warp == kTcCopyWarp && lane == 0) {
       // the latest copy of every stage (earlier ones were consumed)
       const int64_t from = b_issued > S ? b_issued - S : 0;
       for (int64_t gg = from; gg < b_issued; ++gg)
         mbar_wait_drain(&b_full[gg % S], (uint32_t)((gg / S) & 1), status);
     }
-    if (warp == 9 && lane == 0 && mma_tiles > 0) {
+    if (warp == kTcMmaWarp && lane == 0 && mma_tiles > 0) {
       // the last commit completes when every MMA issued before it has
       const int64_t gg = mma_tiles - 1;
       mbar_wait_drain(&b_empty[gg % S], (uint32_t)((gg / S) & 1), status);
@@ -393,6 +419,7 @@ __global__ void __launch_bounds__(kTcThreadsWs, 1)
 constexpr int kSBufs = 4;
 // 16 entry warps in two groups that take alternate tiles (two tiles in flight
 // per row quadrant); group 0 also runs the epilogue.  Then the copy and MMA warps.
+constexpr int kK2tGroup = 256;  // entry threads of a group
 constexpr int kK2tEntry = 512, kK2tThreads = kK2tEntry + 64, kK2tCopyWarp = 16, kK2tMmaWarp = 17;
 constexpr uint32_t kImgVar = 512 * 64;  // one variant of one 512-point image block
 constexpr uint32_t kImgBlock = 4 * kImgVar;
@@ -442,15 +469,15 @@ __global__ void __launch_bounds__(kK2tThreads, 1)
       mbar_init(&b_empty[i], 1);
     }
     for (int i = 0; i < AS; ++i) {
-      mbar_init(&a_full[i], kEntryThreads / 32);
+      mbar_init(&a_full[i], kK2tGroup / 32);
       mbar_init(&a_empty[i], 1);
     }
     for (int i = 0; i < kSBufs; ++i) {
       mbar_init(&s_full[i], 1);
-      mbar_init(&s_empty[i], kEntryThreads / 32);
+      mbar_init(&s_empty[i], kK2tGroup / 32);
     }
     mbar_init(acc_full, 1);
-    mbar_init(acc_empty, kEntryThreads / 32);  // group 0 runs the epilogue
+    mbar_init(acc_empty, kK2tGroup / 32);  // group 0 runs the epilogue
     mbar_init(ar_full, 1);
     mbar_init(ar_empty, 1);
     mbar_init(drain, 1);
@@ -710,6 +737,7 @@ __global__ void k2_reduce_kernel(const float* __restrict__ part, int segs, int64
     const int64_t i = e / k;
     const int q = (int)(e - i * k);
     float s = 0.0f;
+#pragma unroll 8  // the loads of eight segments in flight, added in order
     for (int sg = 0; sg < segs; ++sg) s += part[(int64_t)sg * total + e];
     Y[i * ldy + q] = s + (lam != 0.0f ? lam * X[i * ldx + q] : 0.0f);
   }
@@ -938,16 +966,6 @@ cudaError_t launch_k2(const float* rows32, int64_t m, const float* cols32, int64
 }
 
 cudaError_t set_wait_limit_tc(unsigned long long ns) { return set_wait_limit_this_unit(ns); }
-
-cudaError_t launch_pack_x32(const float* X, int64_t n, int64_t ldx, int k, int N, int64_t ntiles,
-                            uint8_t* img, const int* gate, cudaStream_t s) {
-  const int64_t total = ntiles * 32 * ceil_div(k, N) * N;
-  int64_t g = ceil_div(total, 256);
-  if (g > (int64_t)sm_count() * 16) g = (int64_t)sm_count() * 16;
-  if (g < 1) g = 1;
-  k2_pack_x<32><<<(unsigned)g, 256, 0, s>>>(X, n, ldx, k, N, ntiles, img, gate);
-  return cudaGetLastError();
-}
 
 cudaError_t launch_seg_reduce(const float* part, int segs, int64_t m, int k, float lam,
                               const float* X, int64_t ldx, float* Y, int64_t ldy, const int* gate,

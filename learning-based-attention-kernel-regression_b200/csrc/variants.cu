@@ -47,10 +47,12 @@ int variant_default(int which) {
       if (v >= 0 && v <= 1 << 20) return v;
     }
     // Measured on B200 against the wide kernel (matvec_tc.cu), d = 10 / 16, us:
-    // n = 10,007: k = 48 192 / 197 vs 396 / 468, k = 64 239 / 246 vs 408 / 481,
-    // k = 96 338 / 349 vs 420 / 505, k = 128 426 / 438 vs 424 / 495;
-    // n = 40,000: k = 96 4450 / 4651 vs 4569 / 5653, k = 104 5674 / 5877 vs
-    // 3808 / 4886.
+    // n = 5,003: k = 48 73 / 72 vs 119 / 148, k = 96 114 / 117 vs 131 / 155, k = 104
+    // 139 / 141 vs 109 / 134; n = 10,007: k = 64 234 / 241 vs 346 / 419, k = 96
+    // 329 / 343 vs 338 / 389, k = 128 419 / 438 vs 307 / 385; n = 40,000: k = 64
+    // 2923 / 3064 vs 4723 / 5410, k = 96 4430 / 4646 vs 4167 / 4676, k = 104
+    // 5655 / 5939 vs 3439 / 4472.  65 to 96 is a tie in time and 10 to 100 times
+    // smaller in error here.
     return 96;
   }
   const char* e = getenv("LAKER_K2_LOGITS_TC");
