@@ -120,9 +120,12 @@ __device__ __forceinline__ double exp_tab(double s, const double* __restrict__ s
   q = fma(q, r, 1.0 / 6.0);
   q = fma(q, r, 0.5);
   const double p = fma(r * r, q, r);  // exp(r) - 1
-  const double tj = s_tab[k & 63];
+  // 2^m enters through the table value's exponent field (tj in [1, 2), |m| clamped so
+  // that the field stays normal): one FP64 operation less, the same result
+  const double t0 = s_tab[k & 63];
   const int m = max(-1022, min(1023, k >> 6));
-  return fma(tj, p, tj) * __hiloint2double((m + 1023) << 20, 0);
+  const double tj = __hiloint2double(__double2hiint(t0) + (m << 20), __double2loint(t0));
+  return fma(tj, p, tj);
 }
 
 // ---------------------------------------------------------------------------

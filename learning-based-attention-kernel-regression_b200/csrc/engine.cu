@@ -112,6 +112,52 @@ __device__ __forceinline__ double sum_blocks(const EngineDev& ed, const BlockCtx
   return t;
 }
 
+// Column sums of Q[i][col] * r_i over this warp's rows of the block, for NCH float4
+// chunks per lane.  The loads of RU rows are issued before their FMAs (one row at a
+// time left each row's memory latency exposed: 64 rows per warp and block), the
+// additions stay in row order.
+template <int NCH, int RU>
+__device__ __forceinline__ void project_rows(const float4* __restrict__ Q4, int ldq4,
+                                             const double* __restrict__ r, int64_t seg, int64_t row0,
+                                             int64_t row1, float* __restrict__ s_w) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float4 acc[NCH];
+#pragma unroll
+  for (int ch = 0; ch < NCH; ++ch) acc[ch] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int64_t i0 = row0 + warp; i0 < row1; i0 += (int64_t)NW * RU) {
+    float ri[RU];
+    float4 q[RU][NCH];
+#pragma unroll
+    for (int u = 0; u < RU; ++u) {
+      const int64_t i = i0 + (int64_t)NW * u;
+      const bool ok = i < row1;
+      ri[u] = ok ? (float)r[seg + i] : 0.0f;
+#pragma unroll
+      for (int ch = 0; ch < NCH; ++ch) {
+        const int c4 = lane + 32 * ch;
+        if (ok && c4 < ldq4) q[u][ch] = __ldg(Q4 + i * ldq4 + c4);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < RU; ++u) {
+      if (i0 + (int64_t)NW * u >= row1) break;
+#pragma unroll
+      for (int ch = 0; ch < NCH; ++ch) {
+        if (lane + 32 * ch >= ldq4) continue;
+        acc[ch].x = fmaf(q[u][ch].x, ri[u], acc[ch].x);
+        acc[ch].y = fmaf(q[u][ch].y, ri[u], acc[ch].y);
+        acc[ch].z = fmaf(q[u][ch].z, ri[u], acc[ch].z);
+        acc[ch].w = fmaf(q[u][ch].w, ri[u], acc[ch].w);
+      }
+    }
+  }
+#pragma unroll
+  for (int ch = 0; ch < NCH; ++ch) {
+    const int c4 = lane + 32 * ch;
+    if (c4 < ldq4) reinterpret_cast<float4*>(s_w)[c4] = acc[ch];
+  }
+}
+
 // upart[g][col] = sum over the block's rows i of Q[i][col] * r_i.  Warps take
 // rows; lane l holds the float4 column chunks l + 32 ch.  Caller has
 // synchronised after writing r.
@@ -120,29 +166,10 @@ __device__ void project_block(const EngineDev& ed, const BlockCtx& c, const doub
   const SlotInfo& si = ed.slots[c.k];
   const float4* Q4 = reinterpret_cast<const float4*>(si.q);
   const int ldq = si.ldq, ldq4 = ldq >> 2;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float4 acc[8];
-#pragma unroll
-  for (int ch = 0; ch < 8; ++ch) acc[ch] = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int64_t i = c.row0 + warp; i < c.row1; i += NW) {
-    const float ri = (float)r[c.seg + i];
-#pragma unroll
-    for (int ch = 0; ch < 8; ++ch) {
-      const int c4 = lane + 32 * ch;
-      if (c4 < ldq4) {
-        const float4 q = __ldg(Q4 + i * ldq4 + c4);
-        acc[ch].x = fmaf(q.x, ri, acc[ch].x);
-        acc[ch].y = fmaf(q.y, ri, acc[ch].y);
-        acc[ch].z = fmaf(q.z, ri, acc[ch].z);
-        acc[ch].w = fmaf(q.w, ri, acc[ch].w);
-      }
-    }
-  }
-#pragma unroll
-  for (int ch = 0; ch < 8; ++ch) {
-    const int c4 = lane + 32 * ch;
-    if (c4 < ldq4) reinterpret_cast<float4*>(s_w[warp])[c4] = acc[ch];
-  }
+  float* sw = s_w[threadIdx.x >> 5];
+  if (ldq4 <= 64) project_rows<2, 8>(Q4, ldq4, r, c.seg, c.row0, c.row1, sw);
+  else if (ldq4 <= 128) project_rows<4, 4>(Q4, ldq4, r, c.seg, c.row0, c.row1, sw);
+  else project_rows<8, 2>(Q4, ldq4, r, c.seg, c.row0, c.row1, sw);
   __syncthreads();
   float* dst = ed.upart + c.g * ed.ustride;
   for (int col = threadIdx.x; col < ldq; col += BT) {
@@ -196,13 +223,14 @@ __device__ void w_multiply(const EngineDev& ed, const BlockCtx& c, double* s_u) 
     if (col < nr) {
       const float* wc = W + col;
       int cc = 0;
-      // 16 loads of W issued before their FMAs (same partial sums, same order)
-      for (; cc + 16 <= nr; cc += 16) {
-        float t[16];
+      // 40 loads of W issued before their FMAs (same partial sums, same order)
+      constexpr int WU = 40;
+      for (; cc + WU <= nr; cc += WU) {
+        float t[WU];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) t[e] = __ldg(wc + (int64_t)(cc + e) * nr);
+        for (int e = 0; e < WU; ++e) t[e] = __ldg(wc + (int64_t)(cc + e) * nr);
 #pragma unroll
-        for (int e = 0; e < 16; e += 4) {
+        for (int e = 0; e < WU; e += 4) {
           a0 = fma((double)t[e], s_u[cc + e], a0);
           a1 = fma((double)t[e + 1], s_u[cc + e + 1], a1);
           a2 = fma((double)t[e + 2], s_u[cc + e + 2], a2);
@@ -318,26 +346,45 @@ __global__ void __launch_bounds__(BT)
         constexpr int LPR = decltype(lpr_tag)::value;
         constexpr int RPW = 32 / LPR;
         const int sub = lane / LPR, sl = lane % LPR;
-        for (int64_t i0 = c.row0 + (int64_t)warp * RPW; i0 < c.row1; i0 += (int64_t)NW * RPW) {
-          const int64_t i = i0 + sub;
-          float s = 0.0f;
-          if (i < c.row1) {
-            for (int c4 = sl; c4 < ldq4; c4 += LPR) {
-              const float4 q = __ldg(Q4 + i * ldq4 + c4);
-              const float4 vv = V4[c4];
-              s = fmaf(q.x, vv.x, s);
-              s = fmaf(q.y, vv.y, s);
-              s = fmaf(q.z, vv.z, s);
-              s = fmaf(q.w, vv.w, s);
-            }
+        // two passes of RPW rows at a time, every load of both issued first (8 float4
+        // per lane and pass cover ldq4 <= 8 LPR; a wider row loops)
+        constexpr int PU = 2, CU = 8;
+        for (int64_t i0 = c.row0 + (int64_t)warp * RPW; i0 < c.row1; i0 += (int64_t)NW * RPW * PU) {
+          float s[PU];
+          double ri[PU];
+          float4 q[PU][CU];
+#pragma unroll
+          for (int u = 0; u < PU; ++u) {
+            const int64_t i = i0 + (int64_t)NW * RPW * u + sub;
+            s[u] = 0.0f;
+            ri[u] = i < c.row1 ? r[c.seg + i] : 0.0;
+#pragma unroll
+            for (int t = 0; t < CU; ++t)
+              if (i < c.row1 && sl + LPR * t < ldq4) q[u][t] = __ldg(Q4 + i * ldq4 + sl + LPR * t);
           }
 #pragma unroll
-          for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-          if (sl == 0 && i < c.row1) {
-            const double ri = r[c.seg + i];
-            const float zi = (float)(cis * ri + (double)s);
-            z[c.seg + i] = zi;
-            dot = fma(ri, (double)zi, dot);
+          for (int u = 0; u < PU; ++u) {
+            const int64_t i = i0 + (int64_t)NW * RPW * u + sub;
+            if (i < c.row1) {
+              auto add = [&](const float4& qq, int c4) {
+                const float4 vv = V4[c4];
+                s[u] = fmaf(qq.x, vv.x, s[u]);
+                s[u] = fmaf(qq.y, vv.y, s[u]);
+                s[u] = fmaf(qq.z, vv.z, s[u]);
+                s[u] = fmaf(qq.w, vv.w, s[u]);
+              };
+#pragma unroll
+              for (int t = 0; t < CU; ++t)
+                if (sl + LPR * t < ldq4) add(q[u][t], sl + LPR * t);
+              for (int c4 = sl + LPR * CU; c4 < ldq4; c4 += LPR) add(__ldg(Q4 + i * ldq4 + c4), c4);
+            }
+#pragma unroll
+            for (int o = LPR / 2; o > 0; o >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+            if (sl == 0 && i < c.row1) {
+              const float zi = (float)(cis * ri[u] + (double)s[u]);
+              z[c.seg + i] = zi;
+              dot = fma(ri[u], (double)zi, dot);
+            }
           }
         }
       };
