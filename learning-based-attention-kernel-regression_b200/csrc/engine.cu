@@ -105,11 +105,35 @@ __device__ __forceinline__ void finish_instance(const EngineDev& ed, int k, int 
   ed.done[k] = 1;
 }
 
-// Sum of slot j of the instance's block partials, in block order.
-__device__ __forceinline__ double sum_blocks(const EngineDev& ed, const BlockCtx& c, int j) {
-  double t = 0.0;
-  for (unsigned b = 0; b < c.nblk; ++b) t += __ldcg(ed.bpart + (c.b0 + b) * 4 + j);
-  return t;
+// Sums of the first J slots of the instance's block partials, in block order.  One
+// thread adds them while the instance's other blocks are done, so the loads of 8
+// blocks are issued before their adds.
+template <int J>
+__device__ __forceinline__ void sum_blocks(const EngineDev& ed, const BlockCtx& c, double (&t)[J]) {
+  constexpr int U = 8;
+#pragma unroll
+  for (int j = 0; j < J; ++j) t[j] = 0.0;
+  const double* src = ed.bpart + c.b0 * 4;
+  unsigned b = 0;
+  for (; b + U <= c.nblk; b += U, src += 4 * U) {
+    double v[U][J];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int j = 0; j < J; ++j) v[u][j] = __ldcg(src + 4 * u + j);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int j = 0; j < J; ++j) t[j] += v[u][j];
+  }
+  for (; b < c.nblk; ++b, src += 4)
+#pragma unroll
+    for (int j = 0; j < J; ++j) t[j] += __ldcg(src + j);
+}
+__device__ __forceinline__ double sum_blocks(const EngineDev& ed, const BlockCtx& c) {
+  double t[1];
+  sum_blocks<1>(ed, c, t);
+  return t[0];
 }
 
 // Column sums of Q[i][col] * r_i over this warp's rows of the block, for NCH float4
@@ -130,12 +154,12 @@ __device__ __forceinline__ void project_rows(const float4* __restrict__ Q4, int 
 #pragma unroll
     for (int u = 0; u < RU; ++u) {
       const int64_t i = i0 + (int64_t)NW * u;
-      const bool ok = i < row1;
-      ri[u] = ok ? (float)r[seg + i] : 0.0f;
+      const int64_t ic = i < row1 ? i : row1 - 1;  // rows past the block: loaded, not added
+      ri[u] = (float)r[seg + ic];
 #pragma unroll
       for (int ch = 0; ch < NCH; ++ch) {
         const int c4 = lane + 32 * ch;
-        if (ok && c4 < ldq4) q[u][ch] = __ldg(Q4 + i * ldq4 + c4);
+        if (c4 < ldq4) q[u][ch] = __ldg(Q4 + ic * ldq4 + c4);
       }
     }
 #pragma unroll
@@ -297,7 +321,7 @@ __global__ void __launch_bounds__(BT)
     if (arrive_last_of(&ed.ctr[c.k], c.nblk)) {
       if (threadIdx.x == 0) {
         InstState s{};
-        const double bn = sqrt(sum_blocks(ed, c, 0));
+        const double bn = sqrt(sum_blocks(ed, c));
         s.bnorm = bn;
         s.tol_abs = ed.tol * bn;
         s.rnorm = s.rmax = s.true_rnorm = bn;
@@ -407,7 +431,7 @@ __global__ void __launch_bounds__(BT)
     if (tid == 0) ed.bpart[c.g * 4] = v[0];
     if (arrive_last_of(&ed.ctr[c.k], c.nblk) && tid == 0) {
       InstState& s = ed.st[c.k];
-      const double rz = sum_blocks(ed, c, 0);
+      const double rz = sum_blocks(ed, c);
       s.beta = init ? 0.0 : rz / s.rz;
       s.rz = rz;
       if (!isfinite(rz)) finish_instance(ed, c.k, LAKER_ERR_NONFINITE);
@@ -464,7 +488,9 @@ __global__ void __launch_bounds__(BT)
     }
     if (arrive_last_of(&ed.ctr[c.k], c.nblk) && threadIdx.x == 0) {
       InstState& s = ed.st[c.k];
-      const double pap = sum_blocks(ed, c, 0), pp = sum_blocks(ed, c, 1), aa = sum_blocks(ed, c, 2);
+      double t[3];
+      sum_blocks<3>(ed, c, t);
+      const double pap = t[0], pp = t[1], aa = t[2];
       if (!isfinite(pap) || !isfinite(pp) || !isfinite(aa)) {
         finish_instance(ed, c.k, LAKER_ERR_NONFINITE);
       } else if (pap <= -ed.eps * sqrt(pp) * sqrt(aa)) {
@@ -506,7 +532,7 @@ __global__ void __launch_bounds__(BT)
     if (arrive_last_of(&ed.ctr[c.k], c.nblk)) {
       if (threadIdx.x == 0) {
         InstState& s = ed.st[c.k];
-        const double rn = sqrt(sum_blocks(ed, c, 0));
+        const double rn = sqrt(sum_blocks(ed, c));
         s.rnorm = rn;
         s.iter += 1;
         // replace the residual once the recurrence has fallen by delta from
@@ -555,7 +581,7 @@ __global__ void __launch_bounds__(BT)
     if (arrive_last_of(&ed.ctr[c.k], c.nblk)) {
       if (threadIdx.x == 0) {
         InstState& s = ed.st[c.k];
-        const double rn = sqrt(sum_blocks(ed, c, 0));
+        const double rn = sqrt(sum_blocks(ed, c));
         s.rnorm = s.true_rnorm = s.rmax = rn;
         s.n_accurate += 1;
         s.need_update = 0;

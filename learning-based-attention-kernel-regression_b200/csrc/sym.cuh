@@ -4,6 +4,8 @@
 
 #include <math.h>
 
+#include <type_traits>
+
 #include "internal.cuh"
 
 namespace laker {
@@ -70,28 +72,42 @@ __host__ __device__ inline void sym_pair_coords(int64_t p, int64_t nb, int64_t* 
 // pairs (a' < a, a), in that fixed order.  Both partial arrays hold one
 // B-vector per pair (FP32 kernel: double row sums, float column sums; FP64
 // kernel: both double).
-// The terms go round-robin into four partial sums (independent chains, so
-// the loads overlap), combined as (s0 + s1) + (s2 + s3): a fixed order.
+// The terms go round-robin into four partial sums, combined as
+// (s0 + s1) + (s2 + s3): a fixed order.  Sixteen loads are issued before their
+// adds: a block of the batched engine has few warps, and with four in flight the
+// 40 terms of a 20,000-point instance cost ten memory latencies for each row.
 template <typename RP, typename CP>
 __device__ inline double sym_instance_row_sum(int64_t nb, int64_t ps, int B,
                                               const RP* __restrict__ rowpart,
                                               const CP* __restrict__ colpart, int64_t li) {
   const int64_t a = li / B, o = li - a * B;
-  const int64_t f = ps + sym_first_pair(a, nb);
+  const RP* rp = rowpart + (ps + sym_first_pair(a, nb)) * B + o;
+  const CP* cp = colpart + ps * B + o;
   double s[4] = {0.0, 0.0, 0.0, 0.0};
   const int64_t nq = nb - a;
-  int64_t q = 0;
-  for (; q + 4 <= nq; q += 4) {
+  auto add = [&](auto count, auto load) {
+    constexpr int N = decltype(count)::value;
+    decltype(load(0)) t[N];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) s[u] += (double)rowpart[(f + q + u) * B + o];
-  }
-  for (int u = 0; q < nq; ++q, ++u) s[u] += (double)rowpart[(f + q) * B + o];
-  int64_t ap = 0;
-  for (; ap + 4 <= a; ap += 4) {
+    for (int u = 0; u < N; ++u) t[u] = load(u);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) s[u] += (double)colpart[(ps + sym_pair_index(ap + u, a, nb)) * B + o];
-  }
-  for (int u = 0; ap < a; ++ap, ++u) s[u] += (double)colpart[(ps + sym_pair_index(ap, a, nb)) * B + o];
+    for (int u = 0; u < N; ++u) s[u & 3] += (double)t[u];
+  };
+  auto all = [&](int64_t terms, auto at) {
+    int64_t q = 0;
+    for (; q + 16 <= terms; q += 16) add(std::integral_constant<int, 16>{}, [&](int u) { return at(q + u); });
+    if (q + 8 <= terms) {
+      add(std::integral_constant<int, 8>{}, [&](int u) { return at(q + u); });
+      q += 8;
+    }
+    if (q + 4 <= terms) {
+      add(std::integral_constant<int, 4>{}, [&](int u) { return at(q + u); });
+      q += 4;
+    }
+    for (int u = 0; q < terms; ++q, ++u) s[u] += (double)at(q);
+  };
+  all(nq, [&](int64_t q) { return rp[q * B]; });
+  all(a, [&](int64_t ap) { return cp[sym_pair_index(ap, a, nb) * B]; });
   return (s[0] + s[1]) + (s[2] + s[3]);
 }
 
