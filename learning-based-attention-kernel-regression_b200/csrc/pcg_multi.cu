@@ -41,8 +41,9 @@ namespace {
 constexpr int kMT = 256;         // threads of the vector kernels
 constexpr int kCW = 32;          // columns per CTA of the column-reduction kernels
 constexpr int kRW = kMT / kCW;   // row lanes per CTA
-constexpr int kGT = 64;          // output tile (rows x columns) of the apply's GEMMs
-constexpr int kGK = 16;          // K step of the apply's GEMMs
+constexpr int kGThreads = 128;   // threads of the apply's GEMMs
+constexpr int kGT = 128;         // rows of their output tiles (8 per thread)
+constexpr int kGK = 16;          // their K step
 
 struct alignas(256) MpcgState {
   double bnorm;       // |B|_F
@@ -484,67 +485,113 @@ __global__ void __launch_bounds__(kMT)
 // ---------------------------------------------------------------------------
 namespace {
 
-__global__ void __launch_bounds__(kMT)
+// Tiles of the projection and the expansion: 128 rows x 8 CT columns (CT = 8, 4 or 2,
+// the narrowest that holds the right-hand sides in one tile, 8 when none does), 8 x CT
+// outputs per thread.  The shared-memory loads of the operands bind these GEMMs: with
+// 4 x 4 outputs a thread read two float4 for 16 FMAs (L1 at 79 % of its peak, 138 and
+// 98 us at n = 20,000, N_r = 200, k = 256); 8 x 8 reads
+// four for 64 (106 and 84 us).  k = 16 in 16-column tiles does a quarter of the work of 64
+// (variance of 16 queries at n = 30,011: 241 -> 227 ms).
+
+// acc += A^T B over a K step: a thread's rows are ty 4 .. + 3 and 64 + ty 4 .. + 3, its
+// columns tx 4 .. + 3 and 32 + tx 4 .. + 3 (CT = 8) or tx CT .. + CT - 1.
+template <int CT, int SA, int SB>
+__device__ __forceinline__ void pcm_step(const float (*As)[SA], const float (*Bs)[SB], int ty, int tx,
+                                         float2 (&acc)[8][CT / 2]) {
+#pragma unroll
+  for (int kk = 0; kk < kGK; ++kk) {
+    const float4 a0 = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
+    const float4 a1 = *reinterpret_cast<const float4*>(&As[kk][64 + ty * 4]);
+    const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+    float2 bv[CT / 2];
+    if constexpr (CT == 2) {
+      bv[0] = *reinterpret_cast<const float2*>(&Bs[kk][tx * 2]);
+    } else {
+#pragma unroll
+      for (int h = 0; h < CT / 4; ++h) {
+        const float4 b = *reinterpret_cast<const float4*>(&Bs[kk][h * 32 + tx * 4]);
+        bv[2 * h] = make_float2(b.x, b.y);
+        bv[2 * h + 1] = make_float2(b.z, b.w);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+#pragma unroll
+      for (int v = 0; v < CT / 2; ++v) acc[u][v] = __ffma2_rn(make_float2(av[u], av[u]), bv[v], acc[u][v]);
+  }
+}
+
+__device__ __forceinline__ int pcm_row(int ty, int u) { return (u < 4 ? 0 : 60) + ty * 4 + u; }
+template <int CT>
+__device__ __forceinline__ int pcm_col(int tx, int v) {
+  return CT == 2 ? tx * 2 + v : (v < 4 ? 0 : 28) + tx * 4 + v;
+}
+
+template <int CT>
+__global__ void __launch_bounds__(kGThreads)
     pcm_project_kernel(const float* __restrict__ Q, int ldq, int nq, const double* __restrict__ R,
                        int64_t n, int k, int64_t chunk_rows, double* __restrict__ upart,
                        const int* gate) {
   if (gate && *gate == 0) return;
-  __shared__ __align__(16) float Qs[kGK][kGT];
-  __shared__ __align__(16) float Rs[kGK][kGT];
-  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-  const int j0 = blockIdx.x * kGT, c0 = blockIdx.y * kGT;
+  constexpr int TW = 8 * CT;
+  __shared__ __align__(16) float Qs[2][kGK][kGT];
+  __shared__ __align__(16) float Rs[2][kGK][TW];
+  const int tid = threadIdx.x, tx = tid % 8, ty = tid / 8;
+  const int j0 = blockIdx.x * kGT, c0 = blockIdx.y * TW;
   const int64_t i_begin = (int64_t)blockIdx.z * chunk_rows;
   const int64_t i_end = min(n, i_begin + chunk_rows);
-  float acc[4][4] = {};
-  const int rr = tid / 16, cg = tid % 16;
-  // the next K step's tiles are loaded into registers while this one computes
-  float4 qn;
-  float rn[4];
-  auto fetch = [&](int64_t i) {
-    const int64_t ii = i + rr;
-    const bool row_ok = ii < i_end;
-    const int j = j0 + cg * 4;
-    qn = (row_ok && j < nq) ? *reinterpret_cast<const float4*>(Q + ii * ldq + j)
-                            : make_float4(0.f, 0.f, 0.f, 0.f);
+  float2 acc[8][CT / 2];
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int c = c0 + cg * 4 + v;
-      rn[v] = (row_ok && c < k) ? (float)R[ii * k + c] : 0.0f;
+  for (int u = 0; u < 8; ++u)
+#pragma unroll
+    for (int v = 0; v < CT / 2; ++v) acc[u][v] = make_float2(0.f, 0.f);
+  // the next K step's tiles are loaded into registers while this one computes
+  float4 qn[4];
+  float rn[CT];
+  const int qc = tid % 32 * 4, qr = tid / 32;  // Q: 4 rows at a time, 32 float4 of a row
+  const int rc = tid % TW, rr = tid / TW;      // R: 128 / TW rows at a time
+  const bool q_ok = j0 + qc < nq, r_ok = c0 + rc < k;
+  auto fetch = [&](int64_t i) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int64_t ii = i + qr + 4 * h;
+      qn[h] = (ii < i_end && q_ok) ? *reinterpret_cast<const float4*>(Q + ii * ldq + j0 + qc)
+                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int h = 0; h < CT; ++h) {
+      const int64_t ii = i + rr + (kGThreads / TW) * h;
+      rn[h] = (ii < i_end && r_ok) ? (float)R[ii * k + c0 + rc] : 0.0f;
     }
   };
-  auto store = [&]() {
-    *reinterpret_cast<float4*>(&Qs[rr][cg * 4]) = qn;
+  auto store = [&](int b) {
 #pragma unroll
-    for (int v = 0; v < 4; ++v) Rs[rr][cg * 4 + v] = rn[v];
+    for (int h = 0; h < 4; ++h) *reinterpret_cast<float4*>(&Qs[b][qr + 4 * h][qc]) = qn[h];
+#pragma unroll
+    for (int h = 0; h < CT; ++h) Rs[b][rr + (kGThreads / TW) * h][rc] = rn[h];
   };
   if (i_begin < i_end) {
     fetch(i_begin);
-    store();
+    store(0);
   }
-  for (int64_t i = i_begin; i < i_end; i += kGK) {
+  __syncthreads();
+  int b = 0;
+  for (int64_t i = i_begin; i < i_end; i += kGK, b ^= 1) {
+    const bool more = i + kGK < i_end;
+    if (more) fetch(i + kGK);
+    pcm_step<CT>(Qs[b], Rs[b], ty, tx, acc);
+    if (more) store(b ^ 1);
     __syncthreads();
-    if (i + kGK < i_end) fetch(i + kGK);
-#pragma unroll
-    for (int kk = 0; kk < kGK; ++kk) {
-      const float4 a = *reinterpret_cast<const float4*>(&Qs[kk][ty * 4]);
-      const float4 b = *reinterpret_cast<const float4*>(&Rs[kk][tx * 4]);
-      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(av[u], bv[v], acc[u][v]);
-    }
-    __syncthreads();
-    if (i + kGK < i_end) store();
   }
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int j = j0 + ty * 4 + u;
+  for (int u = 0; u < 8; ++u) {
+    const int j = j0 + pcm_row(ty, u);
     if (j >= nq) continue;
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int c = c0 + tx * 4 + v;
-      if (c < k) upart[((int64_t)blockIdx.z * nq + j) * k + c] = (double)acc[u][v];
+    for (int v = 0; v < CT; ++v) {
+      const int c = c0 + pcm_col<CT>(tx, v);
+      if (c < k)
+        upart[((int64_t)blockIdx.z * nq + j) * k + c] = (double)(v & 1 ? acc[u][v / 2].y : acc[u][v / 2].x);
     }
   }
 }
@@ -601,73 +648,75 @@ __global__ void __launch_bounds__(kMT)
   }
 }
 
-template <typename ZT>
-__global__ void __launch_bounds__(kMT)
+template <int CT, typename ZT>
+__global__ void __launch_bounds__(kGThreads)
     pcm_expand_kernel(const float* __restrict__ Q, int ldq, int nq, int nr,
                       const double* __restrict__ V, const double* __restrict__ R, double cis,
                       int64_t n, int k, ZT* __restrict__ Z, const int* gate) {
   if (gate && *gate == 0) return;
-  __shared__ __align__(16) float Qs[kGK][kGT + 4];  // transposed: Qs[j][i]
-  __shared__ __align__(16) float Vs[kGK][kGT];
-  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+  constexpr int TW = 8 * CT;
+  __shared__ __align__(16) float Qs[2][kGK][kGT + 4];  // transposed: Qs[j][i]
+  __shared__ __align__(16) float Vs[2][kGK][TW];
+  const int tid = threadIdx.x, tx = tid % 8, ty = tid / 8;
   const int64_t i0 = (int64_t)blockIdx.x * kGT;
-  const int c0 = blockIdx.y * kGT;
-  float acc[4][4] = {};
-  // the next K step's tiles are loaded into registers while this one computes
-  const int qi = tid / 4, qg = tid % 4;  // Q tile: 64 rows x 4 groups of 4 columns
-  const int vr = tid / 16, vg = tid % 16;  // V tile: 16 rows x 16 groups of 4 columns
-  float4 qn;
-  float vn[4];
-  auto fetch = [&](int j) {
-    const int64_t i = i0 + qi;
-    const int jc = j + qg * 4;
-    qn = (i < n && jc < nq) ? *reinterpret_cast<const float4*>(Q + i * ldq + jc)
-                            : make_float4(0.f, 0.f, 0.f, 0.f);
-    const int jr = j + vr;
+  const int c0 = blockIdx.y * TW;
+  float2 acc[8][CT / 2];
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int c = c0 + vg * 4 + v;
-      vn[v] = (jr < nr && c < k) ? (float)V[(int64_t)jr * k + c] : 0.0f;
+  for (int u = 0; u < 8; ++u)
+#pragma unroll
+    for (int v = 0; v < CT / 2; ++v) acc[u][v] = make_float2(0.f, 0.f);
+  float4 qn[4];
+  float vn[CT];
+  const int qi = tid / 4, qg = tid % 4 * 4;  // Q: 32 rows at a time, 4 float4 of a row
+  const int vc = tid % TW, vr = tid / TW;    // V: 128 / TW rows at a time
+  const bool v_ok = c0 + vc < k;
+  auto fetch = [&](int j) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int64_t i = i0 + qi + 32 * h;
+      qn[h] = (i < n && j + qg < nq) ? *reinterpret_cast<const float4*>(Q + i * ldq + j + qg)
+                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int h = 0; h < CT; ++h) {
+      const int jr = j + vr + (kGThreads / TW) * h;
+      vn[h] = (jr < nr && v_ok) ? (float)V[(int64_t)jr * k + c0 + vc] : 0.0f;
     }
   };
-  auto store = [&]() {
-    Qs[qg * 4 + 0][qi] = qn.x;
-    Qs[qg * 4 + 1][qi] = qn.y;
-    Qs[qg * 4 + 2][qi] = qn.z;
-    Qs[qg * 4 + 3][qi] = qn.w;
+  auto store = [&](int b) {
 #pragma unroll
-    for (int v = 0; v < 4; ++v) Vs[vr][vg * 4 + v] = vn[v];
+    for (int h = 0; h < 4; ++h) {
+      Qs[b][qg + 0][qi + 32 * h] = qn[h].x;
+      Qs[b][qg + 1][qi + 32 * h] = qn[h].y;
+      Qs[b][qg + 2][qi + 32 * h] = qn[h].z;
+      Qs[b][qg + 3][qi + 32 * h] = qn[h].w;
+    }
+#pragma unroll
+    for (int h = 0; h < CT; ++h) Vs[b][vr + (kGThreads / TW) * h][vc] = vn[h];
   };
   if (nr > 0) {
     fetch(0);
-    store();
+    store(0);
   }
-  for (int j = 0; j < nr; j += kGK) {
+  __syncthreads();
+  int b = 0;
+  for (int j = 0; j < nr; j += kGK, b ^= 1) {
+    const bool more = j + kGK < nr;
+    if (more) fetch(j + kGK);
+    pcm_step<CT>(Qs[b], Vs[b], ty, tx, acc);
+    if (more) store(b ^ 1);
     __syncthreads();
-    if (j + kGK < nr) fetch(j + kGK);
-#pragma unroll
-    for (int kk = 0; kk < kGK; ++kk) {
-      const float4 a = *reinterpret_cast<const float4*>(&Qs[kk][ty * 4]);
-      const float4 b = *reinterpret_cast<const float4*>(&Vs[kk][tx * 4]);
-      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(av[u], bv[v], acc[u][v]);
-    }
-    __syncthreads();
-    if (j + kGK < nr) store();
   }
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int64_t i = i0 + ty * 4 + u;
+  for (int u = 0; u < 8; ++u) {
+    const int64_t i = i0 + pcm_row(ty, u);
     if (i >= n) continue;
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int c = c0 + tx * 4 + v;
+    for (int v = 0; v < CT; ++v) {
+      const int c = c0 + pcm_col<CT>(tx, v);
       if (c < k) {
         const int64_t e = i * k + c;
-        Z[e] = (ZT)(cis * R[e] + (double)acc[u][v]);
+        Z[e] = (ZT)(cis * R[e] + (double)(v & 1 ? acc[u][v / 2].y : acc[u][v / 2].x));
       }
     }
   }
@@ -676,7 +725,10 @@ __global__ void __launch_bounds__(kMT)
 // Columns of Q the apply reads: N_r rounded up to a float4.
 int pcm_cols(int nr) { return (int)round_up(nr, 4); }
 
-int pcm_tiles(int nq, int k) { return (int)(ceil_div(nq, kGT) * ceil_div(k, kGT)); }
+// Columns per thread of the apply's tiles.
+int pcm_ct(int k) { return k <= 16 ? 2 : k <= 32 ? 4 : 8; }
+
+int pcm_tiles(int nq, int k) { return (int)(ceil_div(nq, kGT) * ceil_div(k, 8 * pcm_ct(k))); }
 
 int pcm_chunks(int64_t n, int nq, int k) {
   int64_t c = ceil_div(2 * (int64_t)sm_count(), pcm_tiles(nq, k));
@@ -705,16 +757,18 @@ cudaError_t launch_precond_multi(const laker_precond* pc, const double* R, int k
   double* V = reinterpret_cast<double*>(static_cast<char*>(scratch) +
                                         round_up((int64_t)((size_t)nch * nq * k * sizeof(double)), 256));
   const int64_t chunk_rows = round_up(ceil_div(n, nch), kGK);
-  const unsigned gy = (unsigned)ceil_div(k, kGT);
-  pcm_project_kernel<<<dim3((unsigned)ceil_div(nq, kGT), gy, (unsigned)nch), kMT, 0, s>>>(
-      pc->q_basis, ldq, nq, R, n, k, chunk_rows, upart, gate);
+  const int ct = pcm_ct(k);
+  const unsigned gy = (unsigned)ceil_div(k, 8 * ct);
+  const dim3 pg((unsigned)ceil_div(nq, kGT), gy, (unsigned)nch), eg((unsigned)ceil_div(n, kGT), gy);
+  auto project = ct == 2 ? pcm_project_kernel<2> : ct == 4 ? pcm_project_kernel<4> : pcm_project_kernel<8>;
+  auto expand = ct == 2 ? pcm_expand_kernel<2, ZT> : ct == 4 ? pcm_expand_kernel<4, ZT> : pcm_expand_kernel<8, ZT>;
+  project<<<pg, kGThreads, 0, s>>>(pc->q_basis, ldq, nq, R, n, k, chunk_rows, upart, gate);
   double* U = V + round_up((int64_t)nq * k, 32);
   const int64_t total = (int64_t)nq * k;
   pcm_sum_kernel<<<(unsigned)ceil_div(total, kMT), kMT, 0, s>>>(upart, nch, total, U, gate);
   pcm_core_kernel<<<dim3((unsigned)ceil_div(nq, kCoreJ), (unsigned)ceil_div(k, kCoreC)), kMT, 0, s>>>(
       pc->w_core, nr, nq, U, k, V, gate);
-  pcm_expand_kernel<ZT><<<dim3((unsigned)ceil_div(n, kGT), gy), kMT, 0, s>>>(
-      pc->q_basis, ldq, nq, nr, V, R, pc->inv_sqrt_iso, n, k, Z, gate);
+  expand<<<eg, kGThreads, 0, s>>>(pc->q_basis, ldq, nq, nr, V, R, pc->inv_sqrt_iso, n, k, Z, gate);
   return cudaGetLastError();
 }
 
