@@ -97,7 +97,11 @@ struct ColGrid {
 ColGrid col_grid(int64_t n, int k) {
   ColGrid g{};
   g.gy = (int)ceil_div(k, kCW);
-  int64_t gx = ceil_div(2 * (int64_t)sm_count(), g.gy);
+  // Four CTAs per SM keep more rows in flight (n = 20,000, k = 256: x and r updated in
+  // 41 us, 81 with two CTAs and one row's loads at a time); at most two per SM in one
+  // column group, whose last CTA adds the partial sums of all.
+  int64_t gx = ceil_div(4 * (int64_t)sm_count(), g.gy);
+  if (gx > 2 * (int64_t)sm_count()) gx = 2 * (int64_t)sm_count();
   const int64_t lim = ceil_div(n, kRW);
   if (gx > lim) gx = lim;
   if (gx > 512) gx = 512;
@@ -152,6 +156,7 @@ __device__ __forceinline__ void chunk_totals(const double* bp, int64_t qs, int k
   for (int q = 0; q < NQ; ++q) {
     double t = 0.0;
     if (c < k)
+#pragma unroll 8
       for (unsigned int b = tr; b < gridDim.x; b += kRW) t += __ldcg(bp + q * qs + (int64_t)b * k + c);
     sred[q][tr][tc] = t;
   }
@@ -300,14 +305,29 @@ __global__ void __launch_bounds__(kMT)
   double acc = 0.0;
   if (c < k) {
     const double a = cols.alpha[c];
-#pragma unroll 4  // the loads of four rows in flight
-    for (int64_t i = (int64_t)blockIdx.x * kRW + threadIdx.x / kCW; i < n;
-         i += (int64_t)gridDim.x * kRW) {
-      const int64_t e = i * k + c;
-      X[e] = fma(a, (double)P[e], X[e]);
-      const double r = fma(-a, (double)AP[e], R[e]);
-      R[e] = r;
-      acc = fma(r, r, acc);
+    // four rows at a time, every load before the first store (a store to X or R may
+    // alias the next row's load, so the compiler keeps their order)
+    const int64_t step = (int64_t)gridDim.x * kRW;
+    for (int64_t i = (int64_t)blockIdx.x * kRW + threadIdx.x / kCW; i < n; i += 4 * step) {
+      double x[4], r[4];
+      float p[4], ap[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int64_t e = min(i + u * step, n - 1) * k + c;
+        x[u] = X[e];
+        r[u] = R[e];
+        p[u] = P[e];
+        ap[u] = AP[e];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (i + u * step >= n) break;
+        const int64_t e = (i + u * step) * k + c;
+        X[e] = fma(a, (double)p[u], x[u]);
+        r[u] = fma(-a, (double)ap[u], r[u]);
+        R[e] = r[u];
+        acc = fma(r[u], r[u], acc);
+      }
     }
   }
   const double v[1] = {acc};
@@ -462,11 +482,19 @@ __global__ void __launch_bounds__(kMT)
   if (c >= k) return;
   const bool live = cols.live[c] != 0;
   const float beta = (float)cols.beta[c];
-#pragma unroll 4  // the loads of four rows in flight
-  for (int64_t i = (int64_t)blockIdx.x * kRW + threadIdx.x / kCW; i < n;
-       i += (int64_t)gridDim.x * kRW) {
-    const int64_t e = i * k + c;
-    P[e] = !live ? 0.0f : (init ? Z[e] : fmaf(beta, P[e], Z[e]));
+  const int64_t step = (int64_t)gridDim.x * kRW;
+  for (int64_t i = (int64_t)blockIdx.x * kRW + threadIdx.x / kCW; i < n; i += 4 * step) {
+    float z[4], p[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {  // every load before the first store, as above
+      const int64_t e = min(i + u * step, n - 1) * k + c;
+      z[u] = Z[e];
+      p[u] = init ? 0.0f : P[e];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + u * step < n)
+        P[(i + u * step) * k + c] = !live ? 0.0f : (init ? z[u] : fmaf(beta, p[u], z[u]));
   }
 }
 
