@@ -726,20 +726,36 @@ __global__ void __launch_bounds__(kK2tThreads, 1)
   }
 }
 
-// Y = lam X + sum over segments of the partials, in segment order.
+// Y = lam X + sum over segments of the partials, in segment order.  V columns per
+// thread: 4 (16-byte loads, one division for four) when k is a multiple of 4 and the
+// partials lie on 16 bytes, else 1 (n = 10,000, k = 512: 714 us for the whole product
+// with one column per thread, 686 with four).
+template <int V>
 __global__ void k2_reduce_kernel(const float* __restrict__ part, int segs, int64_t m, int k,
                                  float lam, const float* __restrict__ X, int64_t ldx,
                                  float* __restrict__ Y, int64_t ldy, const int* gate) {
   if (gate && *gate == 0) return;
   const int64_t total = m * (int64_t)k;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t e = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * V; e < total;
+       e += (int64_t)gridDim.x * blockDim.x * V) {
     const int64_t i = e / k;
     const int q = (int)(e - i * k);
-    float s = 0.0f;
+    float s[V] = {};
 #pragma unroll 8  // the loads of eight segments in flight, added in order
-    for (int sg = 0; sg < segs; ++sg) s += part[(int64_t)sg * total + e];
-    Y[i * ldy + q] = s + (lam != 0.0f ? lam * X[i * ldx + q] : 0.0f);
+    for (int sg = 0; sg < segs; ++sg) {
+      if constexpr (V == 4) {
+        const float4 t = *reinterpret_cast<const float4*>(part + (int64_t)sg * total + e);
+        s[0] += t.x;
+        s[1] += t.y;
+        s[2] += t.z;
+        s[3] += t.w;
+      } else {
+        s[0] += part[(int64_t)sg * total + e];
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+      Y[i * ldy + q + v] = s[v] + (lam != 0.0f ? lam * X[i * ldx + q + v] : 0.0f);
   }
 }
 
@@ -959,10 +975,7 @@ cudaError_t launch_k2(const float* rows32, int64_t m, const float* cols32, int64
     LAKER_DISPATCH_TC(dp, e = (launch_k2_tk<DPv, false>(rows32, m, cols32, img, N, TK, wk, lam, X, ldx, k, Y, ldy, part, status, s, gate)));
   }
   if (e != cudaSuccess || wk.segs == 1) return e;
-  int64_t g = ceil_div(m * (int64_t)k, 256);
-  if (g > (int64_t)sm_count() * 16) g = (int64_t)sm_count() * 16;
-  k2_reduce_kernel<<<(unsigned)g, 256, 0, s>>>(part, wk.segs, m, k, lam, X, ldx, Y, ldy, gate);
-  return cudaGetLastError();
+  return launch_seg_reduce(part, wk.segs, m, k, lam, X, ldx, Y, ldy, gate, s);
 }
 
 cudaError_t set_wait_limit_tc(unsigned long long ns) { return set_wait_limit_this_unit(ns); }
@@ -970,10 +983,12 @@ cudaError_t set_wait_limit_tc(unsigned long long ns) { return set_wait_limit_thi
 cudaError_t launch_seg_reduce(const float* part, int segs, int64_t m, int k, float lam,
                               const float* X, int64_t ldx, float* Y, int64_t ldy, const int* gate,
                               cudaStream_t s) {
-  int64_t g = ceil_div(m * (int64_t)k, 256);
+  const bool wide = k % 4 == 0 && reinterpret_cast<uintptr_t>(part) % 16 == 0;
+  int64_t g = ceil_div(m * (int64_t)k, wide ? 1024 : 256);
   if (g > (int64_t)sm_count() * 16) g = (int64_t)sm_count() * 16;
   if (g < 1) g = 1;
-  k2_reduce_kernel<<<(unsigned)g, 256, 0, s>>>(part, segs, m, k, lam, X, ldx, Y, ldy, gate);
+  auto reduce = wide ? k2_reduce_kernel<4> : k2_reduce_kernel<1>;
+  reduce<<<(unsigned)g, 256, 0, s>>>(part, segs, m, k, lam, X, ldx, Y, ldy, gate);
   return cudaGetLastError();
 }
 
