@@ -22,9 +22,12 @@ on packed64 ones; the same tensor passed as rows and cols with m == n selects
 the symmetric operator kernels.  Every op requires CUDA tensors and fails
 loudly otherwise: there is no CPU implementation.
 
-The ops are defined on a torch.library.Library with a CUDA and a fake
-implementation (5 us per call on the host; the same ops through
-torch.library.custom_op took 19 us of a small product's 55).
+The ops are defined on a torch.library.Library (through torch.library.custom_op
+the same ops took 19 us of a small product's 55 on the host, here about 5).  They
+have no gradient formula: the Autograd kernel below attaches a node that refuses
+in the backward pass, eagerly as well as under torch.compile, make_fx and
+torch.func, so that no gradient is lost without an error (the differentiable
+product is AttentionKernelOperator.matvec).
 """
 
 from __future__ import annotations
@@ -38,38 +41,71 @@ from . import _lib
 _LIBRARY = torch.library.Library("laker_b200", "FRAGMENT")
 
 
+# Dispatch keys that follow Autograd, and the context that excludes it.
+_AFTER_AUTOGRAD = torch._C._after_autograd_keyset
+_BelowAutograd = torch._C._AutoDispatchBelowAutograd
+
+
 class _NoBackward(torch.autograd.Function):
     """An op called on tensors that require grad: the result carries a node whose
-    backward refuses (the differentiable product is AttentionKernelOperator.matvec)."""
+    backward refuses.  Without setup_context torch.func's transforms refuse it too."""
 
     @staticmethod
-    def forward(ctx, name, fn, *args):
-        ctx.name = name
-        return fn(*args)
+    def forward(ctx, op, *args):
+        ctx.op = op
+        with _BelowAutograd():
+            return op(*args)
 
     @staticmethod
     def backward(ctx, *grads):
-        raise RuntimeError(f"Trying to backward through laker_b200::{ctx.name} but no autograd "
-                           "formula was registered")
+        raise RuntimeError(f"Trying to backward through {ctx.op} but no autograd formula was "
+                           "registered")
+
+
+def _autograd_kernel(op, fn):
+    """The op's kernel at the Autograd key, which real, fake, functional and
+    torch.func tensors all pass.
+
+    When nothing but the CUDA kernel follows, `fn` is called at once: a second
+    trip through the dispatcher costs 4.5 us.  Which keys follow is read from the
+    call's own keyset (tensors and thread-local modes), so fake tensors, dispatch
+    modes, functionalisation, torch.func levels and lazily negated tensors take
+    the trip."""
+    tensors = tuple(i for i, a in enumerate(op._schema.arguments) if "Tensor" in str(a.type))
+    direct = {}  # keyset -> whether CUDA is the next key, a function of the keyset alone
+    grad_enabled = torch.is_grad_enabled
+
+    def kernel(keyset, *args):
+        if grad_enabled():
+            for i in tensors:
+                if args[i] is not None and args[i].requires_grad:
+                    return _NoBackward.apply(op, *args)
+        raw = keyset.raw_repr()
+        at_once = direct.get(raw)
+        if at_once is None:
+            after = (keyset & _AFTER_AUTOGRAD).highestPriorityTypeId()
+            at_once = direct[raw] = after == torch._C.DispatchKey.CUDA
+        if at_once:
+            return fn(*args)
+        with _BelowAutograd():
+            return op(*args)
+
+    return kernel
 
 
 def _op(schema: str, fake):
-    """Defines laker_b200::<schema>, implemented on CUDA by the decorated function
-    and on fake tensors by `fake`; returns the op overload."""
+    """Defines laker_b200::<schema>, implemented by the decorated function (which
+    refuses tensors that are not on a CUDA device) and on fake tensors by `fake`;
+    returns the op overload."""
     name = schema[: schema.index("(")]
 
     def register(fn):
-        def cuda_impl(*args):
-            if torch.is_grad_enabled() and any(
-                    isinstance(a, torch.Tensor) and a.requires_grad for a in args):
-                return _NoBackward.apply(name, fn, *args)
-            return fn(*args)
-
-        _LIBRARY.define(schema)
-        _LIBRARY.impl(name, cuda_impl, "CUDA")
-        _LIBRARY.impl(name, torch.library.fallthrough_kernel, "Autograd")
+        _LIBRARY.define(schema, tags=(torch.Tag.pt2_compliant_tag,))
+        _LIBRARY.impl(name, fn, "CompositeExplicitAutograd")
         torch.library.register_fake(f"laker_b200::{name}", fake, lib=_LIBRARY)
-        return getattr(torch.ops.laker_b200, name).default
+        op = getattr(torch.ops.laker_b200, name).default
+        _LIBRARY.impl(name, _autograd_kernel(op, fn), "Autograd", with_keyset=True)
+        return op
 
     return register
 
