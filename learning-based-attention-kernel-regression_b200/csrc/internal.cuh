@@ -2,6 +2,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "smem_optin.cuh"
 
 namespace laker {
 

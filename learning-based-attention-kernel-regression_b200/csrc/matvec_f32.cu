@@ -535,13 +535,9 @@ int k1d_rows(int64_t n) {
 template <int DP, int R, bool CLAMP>
 cudaError_t launch_k1d_r(const float* E, int64_t n, float lam, const float* x, float* y, int64_t ldy,
                          int* status, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    const cudaError_t e = cudaFuncSetAttribute(k1d_matvec_f32<DP, R, CLAMP>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static SmemOptIn optin;
+  const cudaError_t e = optin.allow(k1d_matvec_f32<DP, R, CLAMP>, 226 * 1024);
+  if (e != cudaSuccess) return e;
   k1d_matvec_f32<DP, R, CLAMP><<<(unsigned)ceil_div(n, kDWarps * R), kDThreads, k1d_smem_bytes(n, DP), s>>>(
       E, n, lam, x, y, ldy, status);
   return cudaGetLastError();

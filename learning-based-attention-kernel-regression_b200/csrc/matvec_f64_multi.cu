@@ -268,14 +268,9 @@ cudaError_t launch_f64m_t(const double* rows, int64_t m, const double* cols, int
                           const int* gate, cudaStream_t s) {
   constexpr int MT = fm_mt(NT);
   using Cfg = FmCfg<KS, NT, MT>;
-  static bool attr = false;
-  if (!attr) {
-    const cudaError_t e = cudaFuncSetAttribute(f64m_matvec<KS, NT, MT, CLAMP>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)Cfg::kSmem);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static SmemOptIn optin;
+  const cudaError_t e = optin.allow(f64m_matvec<KS, NT, MT, CLAMP>, Cfg::kSmem);
+  if (e != cudaSuccess) return e;
   dim3 grid((unsigned)ceil_div(m, Cfg::kRows), (unsigned)p.chunks, (unsigned)p.S);
   f64m_matvec<KS, NT, MT, CLAMP><<<grid, kFmThreads, Cfg::kSmem, s>>>(
       rows, m, cols, n, DP, lam, X, k, ldx, B, ldb, Y, ldy, p.S > 1 ? part : nullptr,

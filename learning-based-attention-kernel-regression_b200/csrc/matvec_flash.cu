@@ -359,14 +359,9 @@ cudaError_t launch_k2f_t(const uint8_t* rimg, int64_t m, const uint8_t* cimg, co
                          const K2fWork& w, float lam, const float* X, int64_t ldx, int k, float* Y,
                          int64_t ldy, float* part, int* status, const int* gate, cudaStream_t s) {
   using Cfg = K2fCfg<NT>;
-  static bool attr = false;
-  if (!attr) {
-    const cudaError_t e = cudaFuncSetAttribute(k2f_matvec<NT, FMT>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)Cfg::kSmem);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static SmemOptIn optin;
+  const cudaError_t e = optin.allow(k2f_matvec<NT, FMT>, Cfg::kSmem);
+  if (e != cudaSuccess) return e;
   dim3 grid((unsigned)ceil_div(m, Cfg::kRows), (unsigned)w.chunks, (unsigned)w.segs);
   k2f_matvec<NT, FMT><<<grid, kFThreads, Cfg::kSmem, s>>>(rimg, m, cimg, ximg, w.nst, w.sps, lam, X, ldx,
                                                          k, Y, ldy, part, status, gate);

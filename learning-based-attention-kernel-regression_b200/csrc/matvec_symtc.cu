@@ -704,14 +704,9 @@ cudaError_t launch_k1t_t(const uint8_t* img, int64_t n, const float* x, double* 
   using Cfg = K1tCfg<UT, FMT>;
   // the walk's 32-bit pair and point numbers
   if (sp.npairs >= (int64_t)1 << 31 || sp.nb * kTB >= (int64_t)1 << 31) return cudaErrorInvalidValue;
-  static bool attr = false;
-  if (!attr) {
-    const cudaError_t e = cudaFuncSetAttribute(k1t_matvec<UT, FMT, CLAMP, BATCHED>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)Cfg::kSmemBytes);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static SmemOptIn optin;
+  const cudaError_t e = optin.allow(k1t_matvec<UT, FMT, CLAMP, BATCHED>, Cfg::kSmemBytes);
+  if (e != cudaSuccess) return e;
   k1t_matvec<UT, FMT, CLAMP, BATCHED><<<sp.grid, kTThreads, Cfg::kSmemBytes, s>>>(
       img, n, x, colpart, rowpart, sp, bm, status, gate);
   return cudaGetLastError();

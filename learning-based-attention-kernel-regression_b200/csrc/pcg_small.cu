@@ -483,13 +483,9 @@ int small_rows(int64_t n) {
 
 template <int DP, int R>
 cudaError_t launch_small(const SmallArgs& a, int grid, uint32_t smem, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    const cudaError_t e = cudaFuncSetAttribute(pcg_small_kernel<DP, R>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static SmemOptIn optin;
+  const cudaError_t e = optin.allow(pcg_small_kernel<DP, R>, 224 * 1024);
+  if (e != cudaSuccess) return e;
   SmallArgs args = a;
   void* params[] = {&args};
   return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&pcg_small_kernel<DP, R>), dim3(grid),
