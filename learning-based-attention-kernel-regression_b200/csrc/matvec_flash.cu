@@ -8,23 +8,29 @@
 // bound by its chain of hand-offs (MMA -> barrier -> tcgen05.ld -> exp2 ->
 // tcgen05.st -> barrier -> MMA with a nearly empty N): about 230 cycles of an SM
 // sub-partition per 128 entries at k = 16.  Here a warp forms the logits of a 16 x 8
-// tile with two FP16 MMAs, exponentiates the accumulator registers and feeds
-// them straight back as the A operand of the TF32 products, so nothing waits
+// tile with two FP16 MMAs or FP32 FMAs, exponentiates the accumulator registers and
+// feeds them straight back as the A operand of the TF32 products, so nothing waits
 // for another warp; the MMAs themselves are what bounds it (per 128 entries
-// 2 x 8.5 cycles of logits, 25 cycles per 8 right-hand sides; 32 cycles of MUFU
-// ex2 run beside them).
+// 2 x 8.5 cycles of FP16 logits, 25 cycles per 8 right-hand sides; 32 cycles of MUFU
+// ex2 run beside them, 4 d FP32 FMAs a lane only in part).
 //
-// Operands.  Logits: the split-FP16 image of matvec_symtc.cu (kK1tF16x2: V0 W0
-// + V1 W1 = H H' + Hs L' + L Hs'; kK1tF16: (H L' + L H') 2^12 scaled down, then
-// H H').  P X: split TF32, P_hi X_hi + P_hi X_lo + P_lo X_hi, P_hi by truncation,
+// Logits.  Up to 32 right-hand sides: the split-FP16 image of matvec_symtc.cu
+// (kK1tF16x2: V0 W0 + V1 W1 = H H' + Hs L' + L Hs'; kK1tF16: (H L' + L H') 2^12
+// scaled down, then H H'), 22 bits an operand, as the single-RHS operator has it.
+// Above: FP32 FMAs in the order of the wide kernel (matvec_tc.cu), whose products
+// these would otherwise be and which holds the operands in FP32.  22 bits are not
+// enough there: with |e|^2 up to 79 split-FP16 logits cost 3 to 28 times the error
+// (n = 300 .. 30,011: 2e-7 .. 7e-6 with FP32 logits, 2e-6 .. 1.5e-5 without).  FP32
+// logits take 3 to 5 % more time at d = 4, 7 to 24 % at d = 10, 18 to 36 % at d = 16
+// (n from 5,003).  P X: split TF32, P_hi X_hi + P_hi X_lo + P_lo X_hi, P_hi by truncation,
 // the other parts rounded.  The accumulator of a tile holds columns 2t and 2t + 1
 // in lane t where the A operand wants columns t and t + 4: the K index may be
 // taken in any order, so X's rows are stored in that order (k2m_pack_x: one
 // 16-byte load gives a lane its four X values of an 8 x 8 tile).
 //
-// Measured (whole product, before: the tcgen05 form; k = 48 and 64 the wide
-// kernel): n = 50,000, k = 16: 3.44 -> 1.55 ms, k = 32: 3.47 -> 2.45 ms; n = 10,007,
-// k = 16: 188 -> 101 us, k = 64: 405 -> 237 us.  Error against 64 bits, random X:
+// Measured (whole product, before: the tcgen05 form; k = 64 the wide kernel):
+// n = 50,000, k = 16: 3.44 -> 1.55 ms, k = 32: 3.47 -> 2.45 ms; n = 10,007, k = 16:
+// 188 -> 101 us, k = 64: 405 -> 255 us.  Error against 64 bits, random X, |e| up to 2:
 // 6e-5 -> 7e-7 at n = 50,000, 3e-6 -> 7e-7 at n = 10,007.
 //
 // CTA: 8 warps of MT 16-row tiles, one chunk of NT 8-column tiles of right-hand
@@ -45,13 +51,17 @@ constexpr int64_t kFImgBlock = 131072;            // image bytes per 512 points
 constexpr uint32_t kFColVar = kFSlab * 32u;       // a stage's share of a column variant
 constexpr int kFMaxTiles = 8;                     // 8-column tiles of right-hand sides per chunk
 
-// NT tiles of right-hand sides per chunk; MT row tiles per warp.
-template <int NT>
+constexpr int kFMaxF16 = 32;                      // more right-hand sides: FP32 logits
+
+// NT tiles of right-hand sides per chunk; MT row tiles per warp; DP > 0: FP32 logits
+// of DP dimensions.
+template <int NT, int DP>
 struct K2fCfg {
   static constexpr int kMT = NT <= 4 ? 2 : 1;
   static constexpr int kRows = kFWarps * kMT * 16;
   static constexpr uint32_t kXBytes = kFSlab / 8 * NT * 512u;
-  static constexpr uint32_t kStage = 2 * kFColVar + kXBytes;
+  static constexpr uint32_t kColBytes = DP > 0 ? kFSlab * DP * 4u : 2 * kFColVar;
+  static constexpr uint32_t kStage = kColBytes + kXBytes;
   static constexpr int kStages = NT <= 4 ? 4 : 3;
   static constexpr uint32_t kOffBar = kStages * kStage;
   static constexpr uint32_t kSmem = kOffBar + kStages * 8 + 128;  // + alignment slack
@@ -117,15 +127,32 @@ __global__ void k2m_pack_x(const float* __restrict__ X, int64_t n, int64_t ldx, 
   }
 }
 
-template <int NT, int FMT>
+// Column embeddings for FP32 logits: 8-column group, dimension pair h, lane t ->
+// {e[2t][2h], e[2t + 1][2h], e[2t][2h + 1], e[2t + 1][2h + 1]} of the group's points,
+// 16-byte chunks of the packed layout put in the order in which the four lanes of a
+// quad read them (at DP = 16 the packed order has them all on the same banks).
+__global__ void k2m_pack_e(const float4* __restrict__ packed32, int hp, int64_t total,
+                           float4* __restrict__ img, const int* gate) {
+  if (gate && *gate == 0) return;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t q = e >> 2;  // (group, h)
+    const int64_t grp = q / hp;
+    img[e] = packed32[(grp * 4 + (e & 3)) * hp + (q - grp * hp)];
+  }
+}
+
+template <int NT, int FMT, int DP>
 __global__ void __launch_bounds__(kFThreads, 2)
     k2f_matvec(const uint8_t* __restrict__ rimg, int64_t m, const uint8_t* __restrict__ cimg,
                const uint8_t* __restrict__ ximg, int64_t nst, int64_t stages_per_seg, float lam,
                const float* __restrict__ X, int64_t ldx, int k, float* __restrict__ Y, int64_t ldy,
                float* __restrict__ part, int* status, const int* gate) {
   if (gate && *gate == 0) return;
-  using Cfg = K2fCfg<NT>;
+  using Cfg = K2fCfg<NT, DP>;
   constexpr int MT = Cfg::kMT, S = Cfg::kStages;
+  constexpr bool F32 = DP > 0;
+  static_assert(!F32 || MT == 1, "row embeddings in registers");
   constexpr bool X2 = FMT == kK1tF16x2;
   // row operands are variants 0 and 1; the column side starts after the row side
   constexpr uint32_t kColSide = (X2 ? 2u : 3u) * kFVar;
@@ -146,21 +173,35 @@ __global__ void __launch_bounds__(kFThreads, 2)
     const int st = s % S;
     const int64_t gs = s_begin + s, pt = gs * kFSlab;
     uint8_t* dst = sm + st * Cfg::kStage;
-    const uint8_t* src = cimg + (pt / 512) * kFImgBlock + kColSide + (uint32_t)(pt % 512) * 32u;
     mbar_arrive_expect_tx(&full[st], Cfg::kStage);
-    bulk_g2s(dst, src, kFColVar, &full[st]);
-    bulk_g2s(dst + kFColVar, src + kFVar, kFColVar, &full[st]);
-    bulk_g2s(dst + 2 * kFColVar, ximg + ((int64_t)blockIdx.y * nst + gs) * Cfg::kXBytes, Cfg::kXBytes,
+    if constexpr (F32) {
+      bulk_g2s(dst, cimg + gs * Cfg::kColBytes, Cfg::kColBytes, &full[st]);
+    } else {
+      const uint8_t* src = cimg + (pt / 512) * kFImgBlock + kColSide + (uint32_t)(pt % 512) * 32u;
+      bulk_g2s(dst, src, kFColVar, &full[st]);
+      bulk_g2s(dst + kFColVar, src + kFVar, kFColVar, &full[st]);
+    }
+    bulk_g2s(dst + Cfg::kColBytes, ximg + ((int64_t)blockIdx.y * nst + gs) * Cfg::kXBytes, Cfg::kXBytes,
              &full[st]);
   };
   int issued = 0;  // thread 0
   if (tid == 0)
     for (; issued < S - 1 && issued < ns; ++issued) issue(issued);
 
-  // row operands (the image covers whole 512-point blocks, zero past m)
+  // row operands (the image covers whole 512-point blocks, zero past m; FP32: rimg
+  // is the packed layout, whole 256-point tiles)
   const int64_t row0 = (int64_t)blockIdx.x * Cfg::kRows + warp * (MT * 16);
   uint32_t A0[MT][4], A1[MT][4];
-  {
+  float er[2][F32 ? DP : 1];
+  if constexpr (F32) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int64_t r = row0 + g + 8 * h;
+      const float* src = reinterpret_cast<const float*>(rimg) + (r >> 1) * (2 * DP) + (r & 1);
+#pragma unroll
+      for (int q = 0; q < DP; ++q) er[h][q] = r < m ? src[2 * q] * kLog2e : 0.0f;
+    }
+  } else {
     const uint8_t* base = rimg + (row0 / 512) * kFImgBlock;
     const uint32_t r0 = (uint32_t)(row0 % 512) + g;
 #pragma unroll
@@ -187,6 +228,23 @@ __global__ void __launch_bounds__(kFThreads, 2)
 
   // logits of an 8-column group (log2 e folded into the rows)
   auto logits = [&](uint32_t addr, float (&c)[MT][4]) {
+    if constexpr (F32) {
+#pragma unroll
+      for (int h = 0; h < DP / 2; ++h) {
+        float4 v;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr + 64u * h));
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const float e0 = er[u][2 * h], e1 = er[u][2 * h + 1];
+          c[0][2 * u] = h == 0 ? e0 * v.x : fmaf(e0, v.x, c[0][2 * u]);
+          c[0][2 * u + 1] = h == 0 ? e0 * v.y : fmaf(e0, v.y, c[0][2 * u + 1]);
+          c[0][2 * u] = fmaf(e1, v.z, c[0][2 * u]);
+          c[0][2 * u + 1] = fmaf(e1, v.w, c[0][2 * u + 1]);
+        }
+      }
+      return;
+    }
     uint32_t b[4];
     ldmatrix_x4(b, addr);
     const float z[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -207,9 +265,12 @@ __global__ void __launch_bounds__(kFThreads, 2)
       else mma_f16_16816(c[i], A0[i], b[0], b[1], c[i]);
     }
   };
-  // ldmatrix source of this lane: matrix lane / 8 = (variant, chunk), row lane % 8
-  const uint32_t lm_off = (uint32_t)(lane >> 4) * kFColVar +
-                          img16_chunk((uint32_t)(lane & 7), (uint32_t)((lane >> 3) & 1));
+  // ldmatrix source of this lane: matrix lane / 8 = (variant, chunk), row lane % 8;
+  // FP32: the quad lane's chunk of each dimension pair
+  const uint32_t lm_off = F32 ? 16u * t
+                              : (uint32_t)(lane >> 4) * kFColVar +
+                                    img16_chunk((uint32_t)(lane & 7), (uint32_t)((lane >> 3) & 1));
+  constexpr uint32_t kGroup = F32 ? 32u * DP : 256u;  // bytes of an 8-column group
   const uint32_t sm0 = smem_u32(sm) + lm_off;
   bool dead = false;
 #pragma unroll 1
@@ -219,13 +280,13 @@ __global__ void __launch_bounds__(kFThreads, 2)
     __syncthreads();  // every warp has left the stage that is refilled now
     if (tid == 0 && !dead && s + S - 1 < ns) issue(s + S - 1), ++issued;
     const uint32_t ca = sm0 + st * Cfg::kStage;
-    const float4* xb = reinterpret_cast<const float4*>(sm + st * Cfg::kStage + 2 * kFColVar) + lane;
+    const float4* xb = reinterpret_cast<const float4*>(sm + st * Cfg::kStage + Cfg::kColBytes) + lane;
     float c[2][MT][4], acc[MT][NT][4];
     logits(ca, c[0]);
 #pragma unroll
     for (int j = 0; j < kFSlab / 8; ++j) {
       // the next group's logits are issued before this group's exponentials
-      if (j + 1 < kFSlab / 8) logits(ca + (j + 1) * 256u, c[(j + 1) & 1]);
+      if (j + 1 < kFSlab / 8) logits(ca + (j + 1) * kGroup, c[(j + 1) & 1]);
       uint32_t hi[MT][4], lo[MT][4];
 #pragma unroll
       for (int i = 0; i < MT; ++i) {
@@ -354,18 +415,35 @@ K2fLayout k2f_layout(int64_t m, int64_t n, int k, bool same_points) {
 // Largest k that takes this kernel (LAKER_VARIANT_MULTI_FLASH_K; 0 off).
 int k2f_max_k() { return variant_get(LAKER_VARIANT_MULTI_FLASH_K); }
 
-template <int NT, int FMT>
+template <int NT, int FMT, int DP>
 cudaError_t launch_k2f_t(const uint8_t* rimg, int64_t m, const uint8_t* cimg, const uint8_t* ximg,
                          const K2fWork& w, float lam, const float* X, int64_t ldx, int k, float* Y,
                          int64_t ldy, float* part, int* status, const int* gate, cudaStream_t s) {
-  using Cfg = K2fCfg<NT>;
+  using Cfg = K2fCfg<NT, DP>;
   static SmemOptIn optin;
-  const cudaError_t e = optin.allow(k2f_matvec<NT, FMT>, Cfg::kSmem);
+  const cudaError_t e = optin.allow(k2f_matvec<NT, FMT, DP>, Cfg::kSmem);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)ceil_div(m, Cfg::kRows), (unsigned)w.chunks, (unsigned)w.segs);
-  k2f_matvec<NT, FMT><<<grid, kFThreads, Cfg::kSmem, s>>>(rimg, m, cimg, ximg, w.nst, w.sps, lam, X, ldx,
+  k2f_matvec<NT, FMT, DP><<<grid, kFThreads, Cfg::kSmem, s>>>(rimg, m, cimg, ximg, w.nst, w.sps, lam, X, ldx,
                                                          k, Y, ldy, part, status, gate);
   return cudaGetLastError();
+}
+
+// FP32 logits: a chunk has at least five tiles (k > 32), so six or eight.
+template <int DP>
+cudaError_t launch_k2f_f32(const float* rows32, int64_t m, const uint8_t* cimg, const uint8_t* ximg,
+                           const K2fWork& w, float lam, const float* X, int64_t ldx, int k, float* Y,
+                           int64_t ldy, float* part, int* status, const int* gate, cudaStream_t s) {
+  const uint8_t* rows = reinterpret_cast<const uint8_t*>(rows32);
+  switch (w.nt) {
+    case 6:
+      return launch_k2f_t<6, kK1tF16x2, DP>(rows, m, cimg, ximg, w, lam, X, ldx, k, Y, ldy, part,
+                                            status, gate, s);
+    case 8:
+      return launch_k2f_t<8, kK1tF16x2, DP>(rows, m, cimg, ximg, w, lam, X, ldx, k, Y, ldy, part,
+                                            status, gate, s);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 }  // namespace
@@ -393,23 +471,45 @@ cudaError_t launch_k2f(const float* rows32, int64_t m, const float* cols32, int6
   if (g > sm_count() * 8) g = sm_count() * 8;
   k2m_pack_x<<<g, 256, 0, s>>>(X, n, ldx, k, w.nt, w.nst, total, reinterpret_cast<float4*>(ximg), gate);
   cudaError_t e = cudaGetLastError();
-  const int fmt = padded_dim(d) <= 10 ? kK1tF16x2 : kK1tF16;
-  if (e == cudaSuccess) e = launch_k1t_pack(rows32, m, d, rimg, round_up(m, 512), s, fmt);
-  if (e == cudaSuccess && !same) e = launch_k1t_pack(cols32, n, d, cimg, round_up(n, 512), s, fmt);
-  if (e != cudaSuccess) return e;
-  e = cudaErrorInvalidValue;
-  switch (w.nt) {
-#define LAKER_K2F_CASE(W)                                                                           \
-  case W:                                                                                           \
-    e = fmt == kK1tF16x2 ? launch_k2f_t<W, kK1tF16x2>(rimg, m, cimg, ximg, w, lam, X, ldx, k, Y, ldy, \
-                                                      part, status, gate, s)                        \
-                         : launch_k2f_t<W, kK1tF16>(rimg, m, cimg, ximg, w, lam, X, ldx, k, Y, ldy,   \
-                                                    part, status, gate, s);                         \
+  const int dp = padded_dim(d);
+  if (k > kFMaxF16) {
+    if (e != cudaSuccess) return e;
+    const int64_t chunks = w.nst * kFSlab / 2 * (dp / 2);
+    int ge = (int)ceil_div(chunks, 256);
+    if (ge > sm_count() * 8) ge = sm_count() * 8;
+    k2m_pack_e<<<ge, 256, 0, s>>>(reinterpret_cast<const float4*>(cols32), dp / 2, chunks,
+                                  reinterpret_cast<float4*>(cimg), gate);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    e = cudaErrorInvalidValue;
+    switch (dp) {
+#define LAKER_K2F_CASE(D)                                                                            \
+  case D:                                                                                            \
+    e = launch_k2f_f32<D>(rows32, m, cimg, ximg, w, lam, X, ldx, k, Y, ldy, part, status, gate, s);  \
     break;
-    LAKER_K2F_CASE(1) LAKER_K2F_CASE(2) LAKER_K2F_CASE(3) LAKER_K2F_CASE(4) LAKER_K2F_CASE(6)
-    LAKER_K2F_CASE(8)
+      LAKER_K2F_CASE(2) LAKER_K2F_CASE(4) LAKER_K2F_CASE(6) LAKER_K2F_CASE(8) LAKER_K2F_CASE(10)
+      LAKER_K2F_CASE(12) LAKER_K2F_CASE(14) LAKER_K2F_CASE(16)
 #undef LAKER_K2F_CASE
-    default: break;
+      default: break;
+    }
+  } else {
+    const int fmt = dp <= 10 ? kK1tF16x2 : kK1tF16;
+    if (e == cudaSuccess) e = launch_k1t_pack(rows32, m, d, rimg, round_up(m, 512), s, fmt);
+    if (e == cudaSuccess && !same) e = launch_k1t_pack(cols32, n, d, cimg, round_up(n, 512), s, fmt);
+    if (e != cudaSuccess) return e;
+    e = cudaErrorInvalidValue;
+    switch (w.nt) {
+#define LAKER_K2F_CASE(W)                                                                             \
+  case W:                                                                                             \
+    e = fmt == kK1tF16x2 ? launch_k2f_t<W, kK1tF16x2, 0>(rimg, m, cimg, ximg, w, lam, X, ldx, k, Y,    \
+                                                         ldy, part, status, gate, s)                  \
+                         : launch_k2f_t<W, kK1tF16, 0>(rimg, m, cimg, ximg, w, lam, X, ldx, k, Y, ldy, \
+                                                       part, status, gate, s);                        \
+    break;
+      LAKER_K2F_CASE(1) LAKER_K2F_CASE(2) LAKER_K2F_CASE(3) LAKER_K2F_CASE(4)
+#undef LAKER_K2F_CASE
+      default: break;
+    }
   }
   if (e != cudaSuccess || w.segs == 1) return e;
   return launch_seg_reduce(part, w.segs, m, k, lam, X, ldx, Y, ldy, gate, s);

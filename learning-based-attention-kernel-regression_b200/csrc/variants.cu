@@ -47,12 +47,14 @@ int variant_default(int which) {
       if (v >= 0 && v <= 1 << 20) return v;
     }
     // Measured on B200 against the wide kernel (matvec_tc.cu), d = 10 / 16, us:
-    // n = 5,003: k = 48 73 / 72 vs 119 / 148, k = 96 114 / 117 vs 131 / 155, k = 104
-    // 139 / 141 vs 109 / 134; n = 10,007: k = 64 234 / 241 vs 346 / 419, k = 96
-    // 329 / 343 vs 338 / 389, k = 128 419 / 438 vs 307 / 385; n = 40,000: k = 64
-    // 2923 / 3064 vs 4723 / 5410, k = 96 4430 / 4646 vs 4167 / 4676, k = 104
-    // 5655 / 5939 vs 3439 / 4472.  65 to 96 is a tie in time and 10 to 100 times
-    // smaller in error here.
+    // n = 2,500: k = 48 45 / 47 vs 53 / 63, k = 96 55 / 57 vs 57 / 66; n = 5,003: k = 64
+    // 90 / 100 vs 117 / 147, k = 96 129 / 144 vs 123 / 148; n = 10,007: k = 64
+    // 255 / 296 vs 335 / 409, k = 96 392 / 445 vs 329 / 379; n = 40,000: k = 64
+    // 3329 / 3910 vs 4711 / 5386, k = 96 5484 / 6304 vs 4133 / 4639.  So 33 to 64 is
+    // faster here; 65 to 96 is drawn here for its error, which does not grow with n
+    // (6e-7 at every n with |e| up to 2; the wide kernel 1.3e-6 at n = 1,500, 7e-6 at
+    // 12,000, 4e-5 at 30,011), at 0.9 to 1.36 times the wide kernel's time.  From 97 a
+    // third chunk evaluates every entry once more.
     return 96;
   }
   const char* e = getenv("LAKER_K2_LOGITS_TC");
