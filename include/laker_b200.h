@@ -112,7 +112,8 @@ size_t laker_matvec_workspace_bytes(int64_t m, int64_t n, int d, int k, int prec
  * Er/Ec are packed32 buffers of m and n points.  lam is applied only when
  * m == n (pass 0 for a rectangular product such as prediction).  clamp = 1
  * clamps the Gram entry at 80 before exp, as the reference does when
- * max ||e||^2 >= 80.  The n x n kernel matrix is never stored.
+ * max ||e||^2 >= 80.  The n x n kernel matrix is never stored.  With k = 1
+ * the product may be in place (Y == X).
  * Replaces AttentionKernelOperator.matvec / matvec_impl
  * (laker/kernels.py:187-270) and dense_attention_matvec (kernels.py:121-130)
  * for float32 operators. */

@@ -553,6 +553,12 @@ cudaError_t launch_k1d_t(const float* E, int64_t n, float lam, const float* x, f
   }
 }
 
+// Whether [a, a + na) and [b, b + nb) share a byte.
+bool overlap_f32(const float* a, int64_t na, const float* b, int64_t nb) {
+  const uintptr_t ua = reinterpret_cast<uintptr_t>(a), ub = reinterpret_cast<uintptr_t>(b);
+  return ua < ub + (uintptr_t)nb * sizeof(float) && ub < ua + (uintptr_t)na * sizeof(float);
+}
+
 // Whether a square product takes k1d: every point fits a CTA's shared memory and
 // its 16 tiles (the symmetric kernels serve the larger operators).
 bool k1d_fits(int64_t n, int d) {
@@ -696,7 +702,9 @@ extern "C" int laker_attn_matvec_f32(const float* rows32, int64_t m, const float
       e = launch_sym_finish(sp, rowpart, colpart, n, lam, X, Y, ldy, &hdr->status, s);
     return e == cudaSuccess ? LAKER_OK : fail_cuda(e);
   }
-  if (rows32 == cols32 && m == n && k1d_fits(n, d)) {
+  // k1d writes rows while other CTAs still read x: a product in place keeps the
+  // segment kernel, whose finish kernel reads x[i] and then writes y[i]
+  if (rows32 == cols32 && m == n && k1d_fits(n, d) && !overlap_f32(X, n, Y, (n - 1) * ldy + 1)) {
     e = launch_k1d(cols32, n, d, lam, clamp, X, Y, ldy, &hdr->status, s);
     return e == cudaSuccess ? LAKER_OK : fail_cuda(e);
   }
