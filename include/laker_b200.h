@@ -104,7 +104,10 @@ int laker_pack_f64(const void* E, int e_is_f64, int64_t n, int d, int64_t ld, do
 /* Attention-kernel operator                                                 */
 /* ------------------------------------------------------------------------ */
 /* Workspace for laker_attn_matvec_f32 / _f64 (partial row sums of the column
- * segments).  precision is 32 or 64. */
+ * segments).  precision is 32 or 64.  For k > 1 the products also run in less
+ * than this (at least what X and the operand images take, else
+ * LAKER_ERR_WORKSPACE), with fewer column segments: the same sums in another
+ * order.  Partial sums beyond that least size take at most 256 MiB. */
 size_t laker_matvec_workspace_bytes(int64_t m, int64_t n, int d, int k, int precision);
 
 /* FP32 fused matvec ("sloppy" operator used inside the PCG loop).

@@ -50,12 +50,19 @@ cudaError_t launch_multi_f32(const float* rows32, int64_t m, const float* cols32
                              float lam, int clamp, const float* X, int k, int64_t ldx, float* Y,
                              int64_t ldy, cudaStream_t s, const int* gate = nullptr);
 // Y = B - (lam X + K X) when B != nullptr, else lam X + K X (FP64 throughout;
-// matvec_f64_multi.cu).  `part`: f64m_workspace_bytes(m, n, k) of scratch.
-size_t f64m_workspace_bytes(int64_t m, int64_t n, int k);
+// matvec_f64_multi.cu).  `part`: part_bytes of scratch for the partial sums of column
+// segments (may be none); f64m_workspace_bytes is what the product would use of `avail`.
+size_t f64m_workspace_bytes(int64_t m, int64_t n, int k, size_t avail);
 cudaError_t launch_multi_f64(const double* rows64, int64_t m, const double* cols64, int64_t n, int d,
                              double lam, int clamp, const double* X, int k, int64_t ldx,
                              const double* B, int64_t ldb, double* Y, int64_t ldy, double* part,
-                             cudaStream_t s, const int* gate = nullptr);
+                             size_t part_bytes, cudaStream_t s, const int* gate = nullptr);
+
+// Scratch of a multi-RHS product after the header: what a call has to bring (either
+// precision), and what its segments' partial sums may use beyond that where they fill
+// the chip (the products take fewer segments in a smaller workspace).
+size_t multi_min_bytes(int64_t m, int64_t n, int k);
+constexpr size_t kSegScratch = size_t(256) << 20;
 
 // Tensor-core (tcgen05, split TF32) multi-RHS FP32 matvec (matvec_tc.cu).
 int k2_chunk_cols(int k);
@@ -74,12 +81,15 @@ cudaError_t launch_seg_reduce(const float* part, int segs, int64_t m, int k, flo
 
 // ---- flash-style multi-RHS FP32 matvec (matvec_flash.cu) --------------------
 // Whether a product of k right-hand sides takes it (unclamped operators, k up
-// to LAKER_VARIANT_MULTI_FLASH_K), and its workspace.
+// to LAKER_VARIANT_MULTI_FLASH_K), the scratch that it would use of `avail`, and what
+// multi_min_bytes counts for it.
 bool k2f_enabled(int k, int clamp);
-size_t k2f_workspace_bytes(int64_t m, int64_t n, int k, bool same_points);
+size_t k2f_workspace_bytes(int64_t m, int64_t n, int k, bool same_points, size_t avail);
+size_t k2f_reserve_bytes(int64_t m, int64_t n, int k, bool same_points);
 cudaError_t launch_k2f(const float* rows32, int64_t m, const float* cols32, int64_t n, int d,
                        float lam, const float* X, int64_t ldx, int k, float* Y, int64_t ldy,
-                       uint8_t* ws, int* status, cudaStream_t s, const int* gate = nullptr);
+                       uint8_t* ws, size_t ws_bytes, int* status, cudaStream_t s,
+                       const int* gate = nullptr);
 
 // ---- small single-RHS solves in one kernel (pcg_small.cu) ---------------------
 bool pcg_small_fits(int64_t n, int d, int nr, int ldq);

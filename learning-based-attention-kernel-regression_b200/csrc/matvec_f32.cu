@@ -624,19 +624,26 @@ cudaError_t launch_poison_on_status(const int* status, float* Y, int64_t m, int 
   return cudaGetLastError();
 }
 
+size_t multi_min_bytes(int64_t m, int64_t n, int k) {
+  // the tensor-core paths stage X as split, swizzled TF32 tiles (and the
+  // flash-style kernel the operand images of the points)
+  const size_t b = k2_use_tensor_cores() && n > 0 ? (size_t)round_up((int64_t)k2_image_bytes(m, n, k), 256) : 0;
+  const size_t f = n > 0 && m > 0 ? k2f_reserve_bytes(m, n, k, false) : 0;
+  return b > f ? b : f;
+}
+
 }  // namespace laker
 
 using namespace laker;
 
 extern "C" size_t laker_matvec_workspace_bytes(int64_t m, int64_t n, int d, int k, int precision) {
   if (m < 0 || n < 0 || d < 1 || d > 16 || k < 1) return 0;
-  if (k > 1 && precision == 64) return kWsHeader + f64m_workspace_bytes(m, n, k);
   if (k > 1) {
-    // the tensor-core paths stage X as split, swizzled TF32 tiles (and the
-    // flash-style kernel the split-FP16 operand images of the points)
-    size_t b = k2_use_tensor_cores() && n > 0 ? (size_t)round_up((int64_t)k2_image_bytes(m, n, k), 256) : 0;
-    const size_t f = n > 0 && m > 0 ? k2f_workspace_bytes(m, n, k, false) : 0;
-    return kWsHeader + (b > f ? b : f);
+    const size_t least = multi_min_bytes(m, n, k), avail = least > kSegScratch ? least : kSegScratch;
+    size_t use = 0;
+    if (precision == 64) use = f64m_workspace_bytes(m, n, k, avail);
+    else if (m > 0 && n > 0 && k2f_enabled(k, 0)) use = k2f_workspace_bytes(m, n, k, false, avail);
+    return kWsHeader + (use > least ? use : least);
   }
   const SegPlan p = precision == 64 ? k4_plan(m, n, d) : k1_plan(m, n, d);
   size_t bytes = (size_t)p.S * (size_t)m * sizeof(double);
@@ -659,15 +666,20 @@ extern "C" int laker_attn_matvec_f32(const float* rows32, int64_t m, const float
   if (m == 0) return LAKER_OK;
   if (!rows32 || !cols32 || !Y || !workspace || (n > 0 && !X) || (m == n && !X))
     return LAKER_ERR_INVALID_ARG;
-  if (workspace_bytes < laker_matvec_workspace_bytes(m, n, d, k, 32)) return LAKER_ERR_WORKSPACE;
+  if (workspace_bytes < (k > 1 ? kWsHeader + multi_min_bytes(m, n, k)
+                               : laker_matvec_workspace_bytes(m, n, d, k, 32)))
+    return LAKER_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   WsHeader* hdr = static_cast<WsHeader*>(workspace);
   cudaError_t e = cudaMemsetAsync(&hdr->status, 0, sizeof(int), s);
   if (e != cudaSuccess) return fail_cuda(e);
   if (k > 1) {
-    if (n > 0 && k2f_enabled(k, clamp)) {
+    const size_t scratch = workspace_bytes - kWsHeader;
+    // (multi_min_bytes holds the narrow kernel's operands up to k = 192)
+    if (n > 0 && k2f_enabled(k, clamp) &&
+        k2f_workspace_bytes(m, n, k, rows32 == cols32 && m == n, scratch) <= scratch) {
       uint8_t* img = reinterpret_cast<uint8_t*>(workspace) + kWsHeader;
-      e = launch_k2f(rows32, m, cols32, n, d, (m == n) ? lam : 0.0f, X, ldx, k, Y, ldy, img,
+      e = launch_k2f(rows32, m, cols32, n, d, (m == n) ? lam : 0.0f, X, ldx, k, Y, ldy, img, scratch,
                      &hdr->status, s);
       if (e == cudaSuccess) e = launch_poison_on_status(&hdr->status, Y, m, k, ldy, s);
     } else if (k2_use_tensor_cores() && n > 0) {

@@ -211,14 +211,17 @@ extern "C" int laker_attn_matvec_f64(const double* rows64, int64_t m, const doub
   if (m == 0) return LAKER_OK;
   if (!rows64 || !cols64 || !Y || !workspace || (n > 0 && !X) || (m == n && !X))
     return LAKER_ERR_INVALID_ARG;
-  if (workspace_bytes < laker_matvec_workspace_bytes(m, n, d, k, 64)) return LAKER_ERR_WORKSPACE;
+  if (workspace_bytes < (k > 1 ? kWsHeader + multi_min_bytes(m, n, k)
+                               : laker_matvec_workspace_bytes(m, n, d, k, 64)))
+    return LAKER_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   WsHeader* hdr = static_cast<WsHeader*>(workspace);
   cudaError_t e = cudaMemsetAsync(&hdr->status, 0, sizeof(int), s);
   if (e != cudaSuccess) return fail_cuda(e);
   if (k > 1) {
     e = launch_multi_f64(rows64, m, cols64, n, d, (m == n) ? lam : 0.0, clamp, X, k, ldx, B, ldb,
-                         Y, ldy, reinterpret_cast<double*>(static_cast<char*>(workspace) + kWsHeader), s);
+                         Y, ldy, reinterpret_cast<double*>(static_cast<char*>(workspace) + kWsHeader),
+                         workspace_bytes - kWsHeader, s);
     return e == cudaSuccess ? LAKER_OK : fail_cuda(e);
   }
   char* wbase = static_cast<char*>(workspace) + kWsHeader;

@@ -230,7 +230,8 @@ struct FmPlan {
 
 constexpr int fm_mt(int nt) { return nt <= 4 ? 4 : nt <= 8 ? 3 : 2; }
 
-FmPlan f64m_plan(int64_t m, int64_t n, int k) {
+// `avail`: bytes for the segments' partial sums.
+FmPlan f64m_plan(int64_t m, int64_t n, int k, size_t avail) {
   FmPlan p{};
   const int tiles = (k + 7) / 8;
   p.chunks = (tiles + kFmMaxTiles - 1) / kFmMaxTiles;
@@ -246,18 +247,19 @@ FmPlan f64m_plan(int64_t m, int64_t n, int k) {
   // (charged 0.5 % of a segment-free pass, at least 256 columns per segment).
   const int64_t ctas = ceil_div(m > 0 ? m : 1, kFmWarps * p.mt * 8) * p.chunks;
   const int64_t smax = n / 256 < 1 ? 1 : (n / 256 > 16 ? 16 : n / 256);
+  const int64_t nn = n > 0 ? n : 1;
   double best = 1e300;
-  p.S = 1;
   for (int64_t S = 1; S <= smax; ++S) {
     const double cost = (double)ceil_div(ctas * S, sm_count()) / (double)S *
                         (1.0 + 0.005 * (double)(S - 1));
-    if (cost < best - 1e-12) {
+    const int64_t cols = round_up(ceil_div(nn, S), kFmCols), segs = ceil_div(nn, cols);
+    if (cost < best - 1e-12 &&
+        (segs == 1 || (size_t)segs * (size_t)m * (size_t)k * sizeof(double) <= avail)) {
       best = cost;
-      p.S = (int)S;
+      p.S = (int)segs;
+      p.cols_per_seg = cols;
     }
   }
-  p.cols_per_seg = round_up(ceil_div(n > 0 ? n : 1, p.S), kFmCols);
-  p.S = (int)ceil_div(n > 0 ? n : 1, p.cols_per_seg);
   return p;
 }
 
@@ -297,17 +299,17 @@ cudaError_t launch_f64m_nt(const double* rows, int64_t m, const double* cols, in
 
 }  // namespace
 
-size_t f64m_workspace_bytes(int64_t m, int64_t n, int k) {
-  const FmPlan p = f64m_plan(m, n, k);
+size_t f64m_workspace_bytes(int64_t m, int64_t n, int k, size_t avail) {
+  const FmPlan p = f64m_plan(m, n, k, avail);
   return p.S > 1 ? (size_t)p.S * (size_t)m * (size_t)k * sizeof(double) : 0;
 }
 
 cudaError_t launch_multi_f64(const double* rows64, int64_t m, const double* cols64, int64_t n, int d,
                              double lam, int clamp, const double* X, int k, int64_t ldx,
                              const double* B, int64_t ldb, double* Y, int64_t ldy, double* part,
-                             cudaStream_t s, const int* gate) {
+                             size_t part_bytes, cudaStream_t s, const int* gate) {
   if (m <= 0) return cudaSuccess;
-  const FmPlan p = f64m_plan(m, n, k);
+  const FmPlan p = f64m_plan(m, n, k, part_bytes);
   if (p.chunks > 65535) return cudaErrorInvalidValue;
   const int DP = padded_dim(d);
   cudaError_t e = cudaErrorInvalidValue;

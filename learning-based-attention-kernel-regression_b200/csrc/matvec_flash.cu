@@ -368,7 +368,24 @@ struct K2fWork {
 
 constexpr int k2f_rows(int nt) { return kFWarps * (nt <= 4 ? 2 : 1) * 16; }
 
-K2fWork k2f_work(int64_t m, int64_t n, int k) {
+struct K2fLayout {
+  size_t x_off, x_bytes, part_off, rimg_off, cimg_off, total;
+};
+
+K2fLayout k2f_layout(const K2fWork& w, int64_t m, int64_t n, int k, bool same_points) {
+  K2fLayout L{};
+  L.x_off = 0;
+  L.x_bytes = (size_t)w.chunks * (size_t)w.nst * (kFSlab / 8) * (size_t)w.nt * 512;
+  L.part_off = L.x_off + (size_t)round_up((int64_t)L.x_bytes, 1024);
+  const size_t part = w.segs > 1 ? (size_t)w.segs * (size_t)m * (size_t)k * 4 : 0;
+  L.rimg_off = L.part_off + (size_t)round_up((int64_t)part, 1024);
+  L.cimg_off = same_points ? L.rimg_off : L.rimg_off + k1t_image_bytes(m);
+  L.total = L.cimg_off + k1t_image_bytes(n);
+  return L;
+}
+
+// `avail`: bytes of scratch; the segments' partial sums have to fit too.
+K2fWork k2f_work(int64_t m, int64_t n, int k, bool same_points, size_t avail) {
   K2fWork w{};
   const int tiles = (k + 7) / 8;
   w.chunks = (tiles + kFMaxTiles - 1) / kFMaxTiles;
@@ -385,31 +402,19 @@ K2fWork k2f_work(int64_t m, int64_t n, int k) {
   const int64_t slots = 2 * (int64_t)sm_count();
   const int64_t smax = w.nst / 4 < 1 ? 1 : (w.nst / 4 > 32 ? 32 : w.nst / 4);
   double best = 1e300;
-  int segs = 1;
+  auto split = [&](int64_t s) {
+    w.sps = ceil_div(w.nst, s);
+    w.segs = (int)ceil_div(w.nst, w.sps);
+  };
+  int64_t segs = 1;
   for (int64_t s = 1; s <= smax; ++s) {
     const double cost = (double)ceil_div(ctas * s, slots) / (double)s * (1.0 + 0.005 * (double)(s - 1));
-    if (cost < best - 1e-12) best = cost, segs = (int)s;
+    split(s);
+    if (cost < best - 1e-12 && (s == 1 || k2f_layout(w, m, n, k, same_points).total <= avail))
+      best = cost, segs = s;
   }
-  w.sps = ceil_div(w.nst, segs);
-  w.segs = (int)ceil_div(w.nst, w.sps);
+  split(segs);
   return w;
-}
-
-struct K2fLayout {
-  size_t x_off, x_bytes, part_off, rimg_off, cimg_off, total;
-};
-
-K2fLayout k2f_layout(int64_t m, int64_t n, int k, bool same_points) {
-  const K2fWork w = k2f_work(m, n, k);
-  K2fLayout L{};
-  L.x_off = 0;
-  L.x_bytes = (size_t)w.chunks * (size_t)w.nst * (kFSlab / 8) * (size_t)w.nt * 512;
-  L.part_off = L.x_off + (size_t)round_up((int64_t)L.x_bytes, 1024);
-  const size_t part = w.segs > 1 ? (size_t)w.segs * (size_t)m * (size_t)k * 4 : 0;
-  L.rimg_off = L.part_off + (size_t)round_up((int64_t)part, 1024);
-  L.cimg_off = same_points ? L.rimg_off : L.rimg_off + k1t_image_bytes(m);
-  L.total = L.cimg_off + k1t_image_bytes(n);
-  return L;
 }
 
 // Largest k that takes this kernel (LAKER_VARIANT_MULTI_FLASH_K; 0 off).
@@ -450,18 +455,35 @@ cudaError_t launch_k2f_f32(const float* rows32, int64_t m, const uint8_t* cimg, 
 
 bool k2f_enabled(int k, int clamp) { return !clamp && k > 1 && k <= k2f_max_k(); }
 
-size_t k2f_workspace_bytes(int64_t m, int64_t n, int k, bool same_points) {
-  return k2f_layout(m, n, k, same_points).total;
+size_t k2f_workspace_bytes(int64_t m, int64_t n, int k, bool same_points, size_t avail) {
+  return k2f_layout(k2f_work(m, n, k, same_points, avail), m, n, k, same_points).total;
+}
+
+// What every multi-RHS product is given for this kernel, whatever its k: X in chunks
+// of 32 columns, the operand images, partial sums of as many segments as make eight
+// 128-row tiles of a chunk per SM.
+size_t k2f_reserve_bytes(int64_t m, int64_t n, int k, bool same_points) {
+  const int64_t N = round_up(k < 32 ? k : 32, 16), chunks = ceil_div(k, N), slabs = ceil_div(n, kFSlab);
+  const int64_t tiles = ceil_div(m, 128) * chunks, want = 8 * (int64_t)sm_count();
+  int64_t segs = tiles >= want ? 1 : ceil_div(want, tiles);
+  const int64_t most = slabs / 8 > 1 ? slabs / 8 : 1;
+  if (segs > most) segs = most;
+  if (segs > 64) segs = 64;
+  segs = ceil_div(slabs, ceil_div(slabs, segs));
+  const size_t part = segs > 1 ? (size_t)segs * (size_t)m * (size_t)k * 4 : 0;
+  return (size_t)round_up(chunks * slabs * 512 * N, 1024) + (size_t)round_up((int64_t)part, 1024) +
+         (same_points ? 0 : k1t_image_bytes(m)) + k1t_image_bytes(n);
 }
 
 cudaError_t launch_k2f(const float* rows32, int64_t m, const float* cols32, int64_t n, int d,
                        float lam, const float* X, int64_t ldx, int k, float* Y, int64_t ldy,
-                       uint8_t* ws, int* status, cudaStream_t s, const int* gate) {
+                       uint8_t* ws, size_t ws_bytes, int* status, cudaStream_t s, const int* gate) {
   if (m <= 0 || n <= 0 || k < 1) return cudaSuccess;
   const bool same = rows32 == cols32 && m == n;
-  const K2fWork w = k2f_work(m, n, k);
+  const K2fWork w = k2f_work(m, n, k, same, ws_bytes);
   if (w.chunks > 65535) return cudaErrorInvalidValue;
-  const K2fLayout L = k2f_layout(m, n, k, same);
+  const K2fLayout L = k2f_layout(w, m, n, k, same);
+  if (L.total > ws_bytes) return cudaErrorInvalidValue;
   uint8_t* ximg = ws + L.x_off;
   float* part = w.segs > 1 ? reinterpret_cast<float*>(ws + L.part_off) : nullptr;
   uint8_t* rimg = ws + L.rimg_off;

@@ -819,9 +819,9 @@ struct MpcgWs {
   float* AP;
   float* Z;
   double* bp;
-  double* part64;  // segment sums of the FP64 residual (may be empty)
   void* pscratch;
-  uint8_t* img;
+  uint8_t* img;  // operator scratch: FP32 products and, at other times, the FP64 residual
+  size_t img_bytes;
   size_t bytes;
 };
 
@@ -863,13 +863,19 @@ MpcgWs carve_multi(void* base, int64_t n, int k, int nr) {
   w.AP = reinterpret_cast<float*>(take(nk * sizeof(float)));
   w.Z = reinterpret_cast<float*>(take(nk * sizeof(float)));
   w.bp = reinterpret_cast<double*>(take((size_t)3 * g.gx * (size_t)k * sizeof(double)));
-  w.part64 = reinterpret_cast<double*>(take(f64m_workspace_bytes(n, n, k)));
   w.pscratch = nr > 0 ? take(precond_multi_scratch_bytes(n, nr, k)) : nullptr;
   {
     // operator workspace: the tensor-core multi-RHS kernels' operand images
-    const size_t b2 = k2_use_tensor_cores() ? k2_image_bytes(n, n, k) : 0;
-    const size_t bf = k2f_workspace_bytes(n, n, k, true);
-    w.img = reinterpret_cast<uint8_t*>(take(b2 > bf ? b2 : bf));
+    size_t b = k2_use_tensor_cores() ? k2_image_bytes(n, n, k) : 0;
+    const size_t bf = k2f_reserve_bytes(n, n, k, true);
+    if (bf > b) b = bf;
+    const size_t avail = b > kSegScratch ? b : kSegScratch;
+    const size_t u32 = k2f_enabled(k, 0) ? k2f_workspace_bytes(n, n, k, true, avail) : 0;
+    const size_t u64 = f64m_workspace_bytes(n, n, k, avail);
+    if (u32 > b) b = u32;
+    if (u64 > b) b = u64;
+    w.img = reinterpret_cast<uint8_t*>(take(b));
+    w.img_bytes = b;
   }
   w.bytes = off;
   return w;
@@ -912,10 +918,11 @@ int pcg_solve_multi(const laker_operator* op, const laker_precond* pc, const dou
   // R = B - A64 X (gated by `gate`; ungated for the warm start)
   auto launch_residual = [&](int init, const int* gate, cudaStream_t cs) -> cudaError_t {
     cudaError_t ee = launch_multi_f64(op->packed64, n, op->packed64, n, d, op->lambda_reg, op->clamp,
-                                      X, k, k, B, k, w.R, k, w.part64, cs, gate);
+                                      X, k, k, B, k, w.R, k, reinterpret_cast<double*>(w.img),
+                                      w.img_bytes, cs, gate);
     if (ee == cudaSuccess)
       mp_after_residual_kernel<<<cgrid, kMT, 0, cs>>>(w.R, n, k, init, w.bp, w.st, w.cols);
-    launches += f64m_workspace_bytes(n, n, k) > 0 ? 3 : 2;
+    launches += f64m_workspace_bytes(n, n, k, w.img_bytes) > 0 ? 3 : 2;
     return ee;
   };
   auto launch_precond = [&](int init, cudaStream_t cs) -> cudaError_t {
@@ -962,8 +969,8 @@ int pcg_solve_multi(const laker_operator* op, const laker_precond* pc, const dou
   auto iteration = [&](cudaStream_t cs) -> cudaError_t {
     cudaError_t ee;
     if (k2f_enabled(k, op->clamp)) {
-      ee = launch_k2f(op->packed32, n, op->packed32, n, d, lam32, w.P, k, k, w.AP, k, w.img, dstatus,
-                      cs, &w.st->active);
+      ee = launch_k2f(op->packed32, n, op->packed32, n, d, lam32, w.P, k, k, w.AP, k, w.img,
+                      w.img_bytes, dstatus, cs, &w.st->active);
       launches += 4;
     } else if (k2_use_tensor_cores()) {
       ee = launch_k2(op->packed32, n, op->packed32, n, d, op->clamp, lam32, w.P, k, k, w.AP, k, w.img,
