@@ -514,11 +514,10 @@ __global__ void __launch_bounds__(kMT)
 namespace {
 
 // Tiles of the projection and the expansion: 128 rows x 8 CT columns (CT = 8, 4 or 2,
-// the narrowest that holds the right-hand sides in one tile, 8 when none does), 8 x CT
-// outputs per thread.  The shared-memory loads of the operands bind these GEMMs: with
-// 4 x 4 outputs a thread read two float4 for 16 FMAs (L1 at 79 % of its peak, 138 and
-// 98 us at n = 20,000, N_r = 200, k = 256); 8 x 8 reads
-// four for 64 (106 and 84 us).  k = 16 in 16-column tiles does a quarter of the work of 64
+// pcm_ct), 8 x CT outputs per thread.  The shared-memory loads of the operands bind
+// these GEMMs: with 4 x 4 outputs a thread read two float4 for 16 FMAs (L1 at 79 % of
+// its peak, 138 and 98 us at n = 20,000, N_r = 200, k = 256); 8 x 8 reads four for 64
+// (106 and 84 us).  k = 16 in 16-column tiles does a quarter of the work of 64
 // (variance of 16 queries at n = 30,011: 241 -> 227 ms).
 
 // acc += A^T B over a K step: a thread's rows are ty 4 .. + 3 and 64 + ty 4 .. + 3, its
@@ -753,13 +752,27 @@ __global__ void __launch_bounds__(kGThreads)
 // Columns of Q the apply reads: N_r rounded up to a float4.
 int pcm_cols(int nr) { return (int)round_up(nr, 4); }
 
-// Columns per thread of the apply's tiles.
-int pcm_ct(int k) { return k <= 16 ? 2 : k <= 32 ? 4 : 8; }
+// Columns per thread of the apply's tiles.  Wide tiles load less per FMA, but where
+// the expansion has few of them a CTA's chain of steps is what takes the time: a width
+// is passed over for the next only when it gives more than 3 (16 columns) or 4 (32)
+// CTAs per SM.  us at widths 16 / 32 / 64: n = 1,000, N_r = 32, k = 64 23 / 27 / 40;
+// n = 5,000, N_r = 200, k = 64 49 / 55 / 74, k = 200 73 / 64 / 94; n = 20,000,
+// N_r = 200, k = 64 79 / 78 / 90, k = 100 128 / 112 / 119, k = 200 206 / 185 / 185.
+// With 64 columns whenever k > 32 the smallest applies were slower than the 64 x 64
+// tiles before (n = 1,000, N_r = 32, k = 64: 29 us).
+int pcm_ct(int64_t n, int k) {
+  const int64_t rows = ceil_div(n, kGT), sms = sm_count();
+  if (k <= 16 || rows * ceil_div(k, 16) <= 3 * sms) return 2;
+  if (k <= 32 || rows * ceil_div(k, 32) <= 4 * sms) return 4;
+  return 8;
+}
 
-int pcm_tiles(int nq, int k) { return (int)(ceil_div(nq, kGT) * ceil_div(k, 8 * pcm_ct(k))); }
+int pcm_tiles(int64_t n, int nq, int k) {
+  return (int)(ceil_div(nq, kGT) * ceil_div(k, 8 * pcm_ct(n, k)));
+}
 
 int pcm_chunks(int64_t n, int nq, int k) {
-  int64_t c = ceil_div(2 * (int64_t)sm_count(), pcm_tiles(nq, k));
+  int64_t c = ceil_div(2 * (int64_t)sm_count(), pcm_tiles(n, nq, k));
   const int64_t lim = ceil_div(n, 256);
   if (c > lim) c = lim;
   if (c > 64) c = 64;
@@ -785,7 +798,7 @@ cudaError_t launch_precond_multi(const laker_precond* pc, const double* R, int k
   double* V = reinterpret_cast<double*>(static_cast<char*>(scratch) +
                                         round_up((int64_t)((size_t)nch * nq * k * sizeof(double)), 256));
   const int64_t chunk_rows = round_up(ceil_div(n, nch), kGK);
-  const int ct = pcm_ct(k);
+  const int ct = pcm_ct(n, k);
   const unsigned gy = (unsigned)ceil_div(k, 8 * ct);
   const dim3 pg((unsigned)ceil_div(nq, kGT), gy, (unsigned)nch), eg((unsigned)ceil_div(n, kGT), gy);
   auto project = ct == 2 ? pcm_project_kernel<2> : ct == 4 ? pcm_project_kernel<4> : pcm_project_kernel<8>;
