@@ -244,9 +244,14 @@ FmPlan f64m_plan(int64_t m, int64_t n, int k, size_t avail) {
   p.mt = fm_mt(p.nt);
   // Segments: the FP64 pipe is shared by an SM's CTAs, so the time is the most
   // CTAs on an SM over S; each further segment writes and reads m k partial sums
-  // (charged 0.5 % of a segment-free pass, at least 256 columns per segment).
+  // (charged 0.5 % of a segment-free pass, at least 256 columns per segment).  Up to
+  // 511 columns that would be one segment and a few CTAs: there shorter segments fill
+  // the SMs once and no more, as the partial sums weigh more than the entries (n = 300,
+  // k = 500: 58 us in one segment, 23 in four; 51 in the DFMA tiles before).
   const int64_t ctas = ceil_div(m > 0 ? m : 1, kFmWarps * p.mt * 8) * p.chunks;
-  const int64_t smax = n / 256 < 1 ? 1 : (n / 256 > 16 ? 16 : n / 256);
+  int64_t smax = n / (n < 128 ? 32 : n < 512 ? 64 : 256);
+  if (n < 512 && smax > sm_count() / ctas) smax = sm_count() / ctas;
+  smax = smax < 1 ? 1 : (smax > 16 ? 16 : smax);
   const int64_t nn = n > 0 ? n : 1;
   double best = 1e300;
   for (int64_t S = 1; S <= smax; ++S) {
