@@ -81,8 +81,9 @@ __device__ __forceinline__ float ex2_approx(float x) {
 // half the FP64 operations of a general exp: the FP64 operator kernels spend
 // half their time in the exponential.  Each CTA copies the 64-entry table
 // into shared memory (exp_table_to_shared) before its first exp_tab.
-// Results: ~1 ulp for s in [-708, 709]; 2^-1022 ... below (exp gives 0 or a
-// subnormal there), overflow to +inf above; NaN gives NaN.
+// Results: ~1 ulp for s in [-708, 709]; outside m saturates: about 2^-1022 below (exp
+// gives 0 or a subnormal there), a finite value of at least 2^1023 or +inf above; NaN
+// gives NaN.
 // ---------------------------------------------------------------------------
 static __constant__ double c_exp2_64[64] = {
     1.0, 1.0108892860517005, 1.0218971486541166, 1.0330248790212284,
@@ -121,7 +122,8 @@ __device__ __forceinline__ double exp_tab(double s, const double* __restrict__ s
   q = fma(q, r, 0.5);
   const double p = fma(r * r, q, r);  // exp(r) - 1
   // 2^m enters through the table value's exponent field (tj in [1, 2), |m| clamped so
-  // that the field stays normal): one FP64 operation less, the same result
+  // that the field stays normal): one FP64 operation less than a multiplication by 2^m
+  // afterwards, the same bits while the result is normal
   const double t0 = s_tab[k & 63];
   const int m = max(-1022, min(1023, k >> 6));
   const double tj = __hiloint2double(__double2hiint(t0) + (m << 20), __double2loint(t0));
