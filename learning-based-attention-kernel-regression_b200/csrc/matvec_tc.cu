@@ -356,8 +356,8 @@ __global__ void __launch_bounds__(kTcThreadsWs, 1)
         float v[16];
         tmem_ld16(tmem_base + (uint32_t)(ab * 256) + lane_base + (uint32_t)c0, v);
         if (r < m && wk.segs > 1 && (k & 3) == 0 && ch * N + c0 + 16 <= k) {
-          // whole 16-byte chunks of the segment's partial sums (1 KB aligned):
-          // a quarter of the store instructions
+          // whole 16-byte chunks of the segment's partial sums (16-byte aligned, which
+          // launch_k2 checks): a quarter of the store instructions
           float4* dst = reinterpret_cast<float4*>(part + ((int64_t)sg * m + r) * k + ch * N + c0);
 #pragma unroll
           for (int u = 0; u < 4; ++u)
@@ -940,6 +940,8 @@ cudaError_t launch_k2(const float* rows32, int64_t m, const float* cols32, int64
   const K2Work wk = k2_work(m, n, k, N, TK);
   const size_t xbytes = k2_x_image_bytes(wk, N, TK);
   float* part = wk.segs > 1 ? reinterpret_cast<float*>(img + xbytes) : nullptr;
+  // bulk copies from the X image, 16-byte stores of the partial sums
+  if (reinterpret_cast<uintptr_t>(img) % 16 != 0) return cudaErrorMisalignedAddress;
   const size_t pbytes =
       wk.segs > 1 ? (size_t)round_up((int64_t)((size_t)wk.segs * (size_t)m * (size_t)k * 4), 1024) : 0;
   {
