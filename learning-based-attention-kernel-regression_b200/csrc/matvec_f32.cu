@@ -230,9 +230,10 @@ int k1_variant(int dp) {
 // microseconds of arithmetic, and what the segment kernel spends is fill, partial
 // sums and a second launch.  Here every CTA copies all points into shared memory
 // (256-point tiles, one mbarrier each, so the first tile is used while the others
-// arrive; pairs are spread so that no load has bank conflicts), a warp takes R whole rows with its lanes over the column pairs, and the
-// row sum is finished in the warp: no partial sums, no finish kernel.  A lane adds
-// n / 64 pairs in FP32; lanes are added in FP64.
+// arrive; pairs are spread so that no load has bank conflicts), a warp takes R whole
+// rows with its lanes over the column pairs, and the row sum is finished in the warp:
+// no partial sums, no finish kernel.  A lane adds n / 64 pairs in FP32; lanes are
+// added in FP64.
 // n = 1000: the product's C call 18.8 -> 8.2 us on the device (memset + segment
 // kernel + finish before, memset + this kernel now).
 // ---------------------------------------------------------------------------
@@ -316,8 +317,9 @@ __global__ void __launch_bounds__(kDThreads)
 }
 
 // ---------------------------------------------------------------------------
-// Multi-RHS fused FP32 matvec on CUDA cores (LAKER_K2_TC=0, for comparisons):
-// Y = lam X + exp(Er Ec^T) X for X (n x k).  A CTA owns a 64-row x 64-RHS
+// Multi-RHS fused FP32 matvec on CUDA cores (LAKER_K2_TENSOR_CORES=0, for
+// comparisons; unclamped products of up to 96 columns also need
+// LAKER_MULTI_FLASH_K=0): Y = lam X + exp(Er Ec^T) X for X (n x k).  A CTA owns a 64-row x 64-RHS
 // output tile; per 32-column step it evaluates the 64 x 32 block of kernel
 // entries into shared memory (each thread keeps one row embedding in registers,
 // log2 e folded in) and multiplies it into X with 4 x 4 register microtiles.
