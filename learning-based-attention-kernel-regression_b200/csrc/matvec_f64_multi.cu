@@ -74,9 +74,9 @@ struct FmCfg {
 template <int KS, int NT, int MT, bool CLAMP>
 __global__ void __launch_bounds__(kFmThreads, FmCfg<KS, NT, MT>::kMinCtas)
     f64m_matvec(const double* __restrict__ rows, int64_t m, const double* __restrict__ cols,
-                int64_t n, int DP, double lam, const double* __restrict__ X, int k, int64_t ldx,
-                const double* __restrict__ B, int64_t ldb, double* __restrict__ Y, int64_t ldy,
-                double* __restrict__ part, int64_t cols_per_seg, const int* gate) {
+                int64_t n, int DP, int cols16, double lam, const double* __restrict__ X, int k,
+                int64_t ldx, const double* __restrict__ B, int64_t ldb, double* __restrict__ Y,
+                int64_t ldy, double* __restrict__ part, int64_t cols_per_seg, const int* gate) {
   if (gate && *gate == 0) return;
   using Cfg = FmCfg<KS, NT, MT>;
   extern __shared__ __align__(16) double sm[];
@@ -105,7 +105,14 @@ __global__ void __launch_bounds__(kFmThreads, FmCfg<KS, NT, MT>::kMinCtas)
     const int ch = DP >> 1;  // 16-byte chunks of an embedding
     for (int e = tid; e < kFmCols * ch; e += kFmThreads) {
       const int jj = e / ch, c = e - jj * ch;
-      cp_async16(se + jj * Cfg::kLe + 2 * c, cols + (j0 + jj) * DP + 2 * c);
+      double* dst = se + jj * Cfg::kLe + 2 * c;
+      const double* src = cols + (j0 + jj) * DP + 2 * c;
+      if (cols16) {
+        cp_async16(dst, src);
+      } else {  // the caller's buffer lies on 8 bytes
+        cp_async8(dst, src, true);
+        cp_async8(dst + 1, src + 1, true);
+      }
     }
     for (int e = tid; e < kFmCols * NT * 8; e += kFmThreads) {
       const int jj = e / (NT * 8), c = e - jj * (NT * 8);
@@ -282,8 +289,8 @@ cudaError_t launch_f64m_t(const double* rows, int64_t m, const double* cols, int
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)ceil_div(m, Cfg::kRows), (unsigned)p.chunks, (unsigned)p.S);
   f64m_matvec<KS, NT, MT, CLAMP><<<grid, kFmThreads, Cfg::kSmem, s>>>(
-      rows, m, cols, n, DP, lam, X, k, ldx, B, ldb, Y, ldy, p.S > 1 ? part : nullptr,
-      p.cols_per_seg, gate);
+      rows, m, cols, n, DP, reinterpret_cast<uintptr_t>(cols) % 16 == 0, lam, X, k, ldx, B, ldb, Y,
+      ldy, p.S > 1 ? part : nullptr, p.cols_per_seg, gate);
   return cudaGetLastError();
 }
 
@@ -316,6 +323,8 @@ cudaError_t launch_multi_f64(const double* rows64, int64_t m, const double* cols
                              const double* B, int64_t ldb, double* Y, int64_t ldy, double* part,
                              size_t part_bytes, cudaStream_t s, const int* gate) {
   if (m <= 0) return cudaSuccess;
+  // (the partial sums' 16-byte stores; a single segment needs no scratch)
+  if (reinterpret_cast<uintptr_t>(part) % 16 != 0) part_bytes = 0;
   const FmPlan p = f64m_plan(m, n, k, part_bytes);
   if (p.chunks > 65535) return cudaErrorInvalidValue;
   const int DP = padded_dim(d);
