@@ -627,10 +627,11 @@ cudaError_t launch_poison_on_status(const int* status, float* Y, int64_t m, int 
 }
 
 size_t multi_min_bytes(int64_t m, int64_t n, int k) {
+  if (m < 1 || n < 1) return 0;
   // the tensor-core paths stage X as split, swizzled TF32 tiles (and the
   // flash-style kernel the operand images of the points)
-  const size_t b = k2_use_tensor_cores() && n > 0 ? (size_t)round_up((int64_t)k2_image_bytes(m, n, k), 256) : 0;
-  const size_t f = n > 0 && m > 0 ? k2f_reserve_bytes(m, n, k, false) : 0;
+  const size_t b = k2_use_tensor_cores() ? (size_t)round_up((int64_t)k2_image_bytes(m, n, k), 256) : 0;
+  const size_t f = k2f_reserve_bytes(m, n, k, false);
   return b > f ? b : f;
 }
 

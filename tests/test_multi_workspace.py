@@ -52,6 +52,15 @@ def test_product_workspace_is_bounded(precision):
         assert least <= got <= max(least, LIMIT), (m, n, k)
 
 
+@pytest.mark.parametrize("precision", [32, 64])
+def test_empty_products_need_the_header_alone(precision):
+    from laker_b200 import _lib
+
+    for m, n in [(0, 50), (50, 0), (0, 0)]:
+        for k in (2, 40, 300):
+            assert _lib.load().laker_matvec_workspace_bytes(m, n, 4, k, precision) == HEADER
+
+
 def test_solve_workspace_is_bounded():
     from laker_b200 import _lib
 
