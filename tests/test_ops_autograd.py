@@ -81,3 +81,34 @@ def test_tracing_without_gradients():
 def test_cpu_tensors_name_the_device_that_is_wanted():
     with pytest.raises(RuntimeError, match="must be a CUDA tensor"):
         OPS.pack(torch.zeros(4, 3), 32)
+
+
+@pytest.mark.gpu
+def test_cuda_tensors_that_may_not_skip_the_dispatcher(cuda):
+    """Lazily negated tensors, vmap and dispatch modes on real tensors give what plain
+    ones give; torch.func.grad refuses."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    g = torch.Generator(device=cuda).manual_seed(0)
+    p = OPS.pack(torch.randn(N, D, generator=g, device=cuda) * 0.5, 32)
+    X = torch.randn(3, N, generator=g, device=cuda)
+    one = lambda t: OPS.attn_matvec(p, N, p, N, D, 0.1, False, t)  # noqa: E731
+    want = torch.stack([one(t) for t in X])
+    neg = torch.complex(X[0], X[1]).conj().imag  # a view with the negative bit: -X[1]
+    assert neg.is_neg()
+    assert torch.equal(one(neg), one((-X[1]).contiguous()))
+    assert torch.equal(torch.func.vmap(one)(X), want)
+    seen = []
+
+    class Names(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    with Names():
+        y = one(X[0])
+    assert torch.equal(y, want[0]) and "laker_b200.attn_matvec.default" in seen
+    with torch.inference_mode():
+        assert torch.equal(one(X[0]), want[0])
+    with pytest.raises(RuntimeError, match="setup_context"):
+        torch.func.grad(lambda t: (one(t) + t).sum())(X[0])
