@@ -71,12 +71,14 @@ struct FmCfg {
   static constexpr int kMinCtas = MT * NT >= 26 ? 2 : 3;
 };
 
-template <int KS, int NT, int MT, bool CLAMP>
+// A16: the column embeddings lie on 16 bytes (else they are copied 8 at a time; a
+// choice at run time cost 4.6 % at 16 tiles, n = 20,000, k = 256).
+template <int KS, int NT, int MT, bool CLAMP, bool A16>
 __global__ void __launch_bounds__(kFmThreads, FmCfg<KS, NT, MT>::kMinCtas)
     f64m_matvec(const double* __restrict__ rows, int64_t m, const double* __restrict__ cols,
-                int64_t n, int DP, int cols16, double lam, const double* __restrict__ X, int k,
-                int64_t ldx, const double* __restrict__ B, int64_t ldb, double* __restrict__ Y,
-                int64_t ldy, double* __restrict__ part, int64_t cols_per_seg, const int* gate) {
+                int64_t n, int DP, double lam, const double* __restrict__ X, int k, int64_t ldx,
+                const double* __restrict__ B, int64_t ldb, double* __restrict__ Y, int64_t ldy,
+                double* __restrict__ part, int64_t cols_per_seg, const int* gate) {
   if (gate && *gate == 0) return;
   using Cfg = FmCfg<KS, NT, MT>;
   extern __shared__ __align__(16) double sm[];
@@ -107,9 +109,9 @@ __global__ void __launch_bounds__(kFmThreads, FmCfg<KS, NT, MT>::kMinCtas)
       const int jj = e / ch, c = e - jj * ch;
       double* dst = se + jj * Cfg::kLe + 2 * c;
       const double* src = cols + (j0 + jj) * DP + 2 * c;
-      if (cols16) {
+      if constexpr (A16) {
         cp_async16(dst, src);
-      } else {  // the caller's buffer lies on 8 bytes
+      } else {
         cp_async8(dst, src, true);
         cp_async8(dst + 1, src + 1, true);
       }
@@ -231,6 +233,7 @@ __global__ void f64m_reduce_kernel(const double* __restrict__ part, int S, int64
 // 1.5 times apart from 4 on, 1.3 times from 8 on (every absent tile of a chunk costs
 // as much as a present one); each further width is eight more kernels to build.
 constexpr int kFmWidths[] = {1, 2, 4, 6, 8, 10, 13, 16};
+constexpr int kFmOddWidth = 4;
 
 struct FmPlan {
   int nt, mt, chunks, S;
@@ -239,8 +242,9 @@ struct FmPlan {
 
 constexpr int fm_mt(int nt) { return nt <= 4 ? 4 : nt <= 8 ? 3 : 2; }
 
-// `avail`: bytes for the segments' partial sums.
-FmPlan f64m_plan(int64_t m, int64_t n, int k, size_t avail) {
+// `avail`: bytes for the segments' partial sums.  `a16`: whether the column embeddings
+// lie on 16 bytes; where they do not, one width serves every k.
+FmPlan f64m_plan(int64_t m, int64_t n, int k, size_t avail, bool a16 = true) {
   FmPlan p{};
   const int tiles = (k + 7) / 8;
   p.chunks = (tiles + kFmMaxTiles - 1) / kFmMaxTiles;
@@ -250,6 +254,10 @@ FmPlan f64m_plan(int64_t m, int64_t n, int k, size_t avail) {
       p.nt = w;
       break;
     }
+  if (!a16) {
+    p.nt = kFmOddWidth;
+    p.chunks = (tiles + kFmOddWidth - 1) / kFmOddWidth;
+  }
   p.mt = fm_mt(p.nt);
   // Segments: the FP64 pipe is shared by an SM's CTAs, so the time is the most
   // CTAs on an SM over S; each further segment writes and reads m k partial sums
@@ -277,7 +285,7 @@ FmPlan f64m_plan(int64_t m, int64_t n, int k, size_t avail) {
   return p;
 }
 
-template <int KS, int NT, bool CLAMP>
+template <int KS, int NT, bool CLAMP, bool A16 = true>
 cudaError_t launch_f64m_t(const double* rows, int64_t m, const double* cols, int64_t n, int DP,
                           double lam, const double* X, int k, int64_t ldx, const double* B,
                           int64_t ldb, double* Y, int64_t ldy, double* part, const FmPlan& p,
@@ -285,12 +293,12 @@ cudaError_t launch_f64m_t(const double* rows, int64_t m, const double* cols, int
   constexpr int MT = fm_mt(NT);
   using Cfg = FmCfg<KS, NT, MT>;
   static SmemOptIn optin;
-  const cudaError_t e = optin.allow(f64m_matvec<KS, NT, MT, CLAMP>, Cfg::kSmem);
+  const cudaError_t e = optin.allow(f64m_matvec<KS, NT, MT, CLAMP, A16>, Cfg::kSmem);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)ceil_div(m, Cfg::kRows), (unsigned)p.chunks, (unsigned)p.S);
-  f64m_matvec<KS, NT, MT, CLAMP><<<grid, kFmThreads, Cfg::kSmem, s>>>(
-      rows, m, cols, n, DP, reinterpret_cast<uintptr_t>(cols) % 16 == 0, lam, X, k, ldx, B, ldb, Y,
-      ldy, p.S > 1 ? part : nullptr, p.cols_per_seg, gate);
+  f64m_matvec<KS, NT, MT, CLAMP, A16><<<grid, kFmThreads, Cfg::kSmem, s>>>(
+      rows, m, cols, n, DP, lam, X, k, ldx, B, ldb, Y, ldy, p.S > 1 ? part : nullptr,
+      p.cols_per_seg, gate);
   return cudaGetLastError();
 }
 
@@ -299,6 +307,9 @@ cudaError_t launch_f64m_nt(const double* rows, int64_t m, const double* cols, in
                            double lam, const double* X, int k, int64_t ldx, const double* B,
                            int64_t ldb, double* Y, int64_t ldy, double* part, const FmPlan& p,
                            const int* gate, cudaStream_t s) {
+  if (reinterpret_cast<uintptr_t>(cols) % 16 != 0)
+    return launch_f64m_t<KS, kFmOddWidth, CLAMP, false>(rows, m, cols, n, DP, lam, X, k, ldx, B, ldb, Y,
+                                                        ldy, part, p, gate, s);
   switch (p.nt) {
 #define LAKER_FM_CASE(W)                                                                         \
   case W:                                                                                        \
@@ -325,7 +336,7 @@ cudaError_t launch_multi_f64(const double* rows64, int64_t m, const double* cols
   if (m <= 0) return cudaSuccess;
   // (the partial sums' 16-byte stores; a single segment needs no scratch)
   if (reinterpret_cast<uintptr_t>(part) % 16 != 0) part_bytes = 0;
-  const FmPlan p = f64m_plan(m, n, k, part_bytes);
+  const FmPlan p = f64m_plan(m, n, k, part_bytes, reinterpret_cast<uintptr_t>(cols64) % 16 == 0);
   if (p.chunks > 65535) return cudaErrorInvalidValue;
   const int DP = padded_dim(d);
   cudaError_t e = cudaErrorInvalidValue;
