@@ -233,7 +233,8 @@ int laker_noalloc_status(int* status, void* stream);
  * FP64 accumulation).
  *   Y = B - (lam * X[:m] + exp(Er Ec^T) X)    if B != NULL
  *   Y =      lam * X[:m] + exp(Er Ec^T) X     otherwise
- * Er/Ec are packed64 buffers.  Used for the true-residual recomputation of
+ * Er/Ec are packed64 buffers.  With k = 1 the product may be in place (Y == X).
+ * Used for the true-residual recomputation of
  * the PCG loop and for float64 operators and predictions.
  * Replaces the float64 path of AttentionKernelOperator.matvec
  * (laker/kernels.py:187-270), the residual replacement r = b - A x

@@ -16,8 +16,8 @@
 //
 // Measured (whole product; before: 64 x 64 tiles of DFMA microtiles with the
 // entries in shared memory, bound by its shared-memory loads and barriers):
-// n = 20,000, k = 512: 37.8 -> 18.0 ms (0.72 of the FP64 pipe's rate);
-// n = 8,009, k = 200: 3.60 -> 1.27 ms; n = 30,011, k = 16: 2.5 ms (0.76).  Error
+// n = 20,000, k = 512: 37.8 -> 17.6 ms (0.73 of the FP64 pipe's rate);
+// n = 8,009, k = 200: 3.61 -> 1.23 ms; n = 30,011, k = 16: 2.5 ms (0.76).  Error
 // against 64-bit torch at n = 8,009, k = 200: 3.1e-15 -> 1.9e-15.
 //
 // CTA: 4 warps, 32 MT rows, one chunk of NT 8-column tiles of right-hand sides

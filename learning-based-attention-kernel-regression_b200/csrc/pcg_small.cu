@@ -20,7 +20,7 @@
 // Precision: as pcg.cu (FP32 entries, p, z, Ap; FP64 x, r, dots, residuals); the
 // preconditioner is applied in FP64 from the FP32 factors (pcg.cu: FP32 products).
 //
-// n = 2000 (N_r = 200, tol 1e-10): 18.5 -> 6.4 ms, 66 -> 19 us per iteration; n = 500:
+// n = 2000 (N_r = 200, tol 1e-10): 18.0 -> 6.4 ms, 66 -> 19 us per iteration; n = 500:
 // 12 us, n = 3000: 24 us.  About 10 us of an iteration is the chain of four barriers and
 // the L2 round trips between them (a 40-point solve takes that), the rest the operator
 // on the CUDA cores (6 us at n = 3000).  Measured the same: 16 warps per CTA, three rows

@@ -61,3 +61,20 @@ def test_outputs_that_only_touch_the_input(cuda):
                                              Y.data_ptr(), 1, ws.data_ptr(), ws.numel(),
                                              _lib.stream_handle(torch.device(cuda))), "matvec")
         assert torch.equal(Y, want) and torch.equal(X, x)
+
+
+@pytest.mark.parametrize("n,d", [(1, 10), (300, 10), (3500, 4)])
+def test_f64_product_in_place(cuda, n, d):
+    from laker_b200 import _lib
+
+    lib = _lib.load()
+    rng = np.random.default_rng(n)
+    E, x = rng.standard_normal((n, d)) / np.sqrt(d), rng.standard_normal(n)
+    p = _lib.pack_f64(torch.tensor(E, device=cuda))
+    want = _lib.attn_matvec_f64(p, n, p, n, d, 0.1, 0, torch.tensor(x, device=cuda))
+    ws = _lib.workspace(lib.laker_matvec_workspace_bytes(n, n, d, 1, 64), torch.device(cuda))
+    buf = torch.tensor(x, device=cuda)
+    _lib.check(lib.laker_attn_matvec_f64(p.data_ptr(), n, p.data_ptr(), n, d, 0.1, 0, buf.data_ptr(), 1, 1, None, 1,
+                                         buf.data_ptr(), 1, ws.data_ptr(), ws.numel(),
+                                         _lib.stream_handle(torch.device(cuda))), "matvec")
+    assert torch.equal(buf, want)
