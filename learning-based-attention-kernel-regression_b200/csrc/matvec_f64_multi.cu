@@ -266,7 +266,8 @@ FmPlan f64m_plan(int64_t m, int64_t n, int k, size_t avail, bool a16 = true) {
   // the SMs once and no more, as the partial sums weigh more than the entries (n = 300,
   // k = 500: 58 us in one segment, 23 in four; 51 in the DFMA tiles before).
   const int64_t ctas = ceil_div(m > 0 ? m : 1, kFmWarps * p.mt * 8) * p.chunks;
-  int64_t smax = n / (n < 128 ? 32 : n < 512 ? 64 : 256);
+  const bool wide = p.nt >= 10;  // below 128 columns the sum's launch pays only there
+  int64_t smax = n / (n < 128 && wide ? 32 : n < 512 ? 64 : 256);
   if (n < 512 && smax > sm_count() / ctas) smax = sm_count() / ctas;
   smax = smax < 1 ? 1 : (smax > 16 ? 16 : smax);
   const int64_t nn = n > 0 ? n : 1;

@@ -1,6 +1,6 @@
 """FP64 multi-RHS products over few columns (csrc/matvec_f64_multi.cu): up to 511 they
-are cut into segments of at least 32 (below 128) or 64 columns while the CTAs fit the
-SMs once.  Both sides of each line, full and ragged segments, squares and rectangles,
+are cut into segments of at least 64 columns (32 below 128 and above 64 right-hand
+sides) while the CTAs fit the SMs once.  Both sides of each line, full and ragged segments, squares and rectangles,
 against the float64 oracle.  Tolerance as for the tiles: an entry's logit rounds by
 (d + 1) eps sum |e_ik e_jk|, its exp by 2 ulp, the sum by n eps, twice for the oracle.
 """
